@@ -80,13 +80,16 @@ BYTES_PER_NODE = 80
 # `traffic` and its issue-bound floor (warp instructions / (4 schedulers x
 # SMs x SM clock)).
 NCU_KERNELS = {
-    "k_subblocks": {"dram_bytes": 4203264, "warp_inst": 1975877},
-    "k_stress": {"dram_bytes": 195174912 + 62206208, "warp_inst": 39083888},
-    "k_bounds": {"dram_bytes": 4864, "warp_inst": 172},
-    "k_p2g_tiles": {"dram_bytes": 96181760 + 5001984, "warp_inst": 56973418},
+    "k_count": {"dram_bytes": None, "warp_inst": None},
+    "k_offsets": {"dram_bytes": None, "warp_inst": None},
+    "k_place": {"dram_bytes": None, "warp_inst": None},
+    "k_rank": {"dram_bytes": None, "warp_inst": None},
+    "k_stress": {"dram_bytes": None, "warp_inst": None},
+    "k_p2g_sweep": {"dram_bytes": None, "warp_inst": None},
     "k_g2p": {"dram_bytes": 54698240 + 46928640, "warp_inst": 53436416},
 }
-P2G_KERNELS = ("k_subblocks", "k_stress", "k_bounds", "k_p2g_tiles")
+P2G_KERNELS = ("k_count", "k_offsets", "k_place", "k_rank", "k_stress", "k_p2g_sweep")
+LAUNCHES_PER_SUBSTEP = 3 + len(P2G_KERNELS)   # and clock, grid, g2p; one scene or a batch of any number
 
 
 def parse():
@@ -197,7 +200,7 @@ def build_sim(torch, device, seed):
 
 
 def time_kernels(torch, sim, steps, t0):
-    """Per-kernel device time (ms per launch) via events around each C-ABI piece."""
+    """Device time (ms per substep) of each phase via events around its C-ABI piece (P2G with its binning)."""
     from peel_mpm_b200 import _lib
     grips, _ = sim._descriptors()
     prm = sim._build_params(grips)
@@ -206,24 +209,22 @@ def time_kernels(torch, sim, steps, t0):
     s = torch.cuda.current_stream()
     sp = s.cuda_stream
     ws, nb = sim._ws.data_ptr(), sim._ws_bytes
-    names = ["bin", "p2g", "grid", "g2p"]
+    names = ["p2g", "grid", "g2p"]
     acc = {k: 0.0 for k in names}
     for i in range(steps):
-        ev = [torch.cuda.Event(enable_timing=True) for _ in range(5)]
+        ev = [torch.cuda.Event(enable_timing=True) for _ in range(4)]
         clk = sim._clock(t0 + i * sim.dt, sim._step)
-        ev[0].record(s)
         _lib.check(lib.pm_set_clock(C.byref(prm), ws, nb, sim.n, C.byref(clk), sp))
-        _lib.check(lib.pm_bin(C.byref(prm), C.byref(P), ws, nb, sp))
-        ev[1].record(s)
+        ev[0].record(s)
         _lib.check(lib.pm_p2g(C.byref(prm), C.byref(P), ws, nb, sp))
-        ev[2].record(s)
+        ev[1].record(s)
         _lib.check(lib.pm_grid_update(C.byref(prm), ws, nb, sim.n, sp))
-        ev[3].record(s)
+        ev[2].record(s)
         _lib.check(lib.pm_g2p(C.byref(prm), C.byref(P), ws, nb, sp))
-        ev[4].record(s)
+        ev[3].record(s)
         sim._step += 1
         torch.cuda.synchronize()
-        for k in range(4):
+        for k in range(3):
             acc[names[k]] += ev[k].elapsed_time(ev[k + 1])
     return {k: v / steps for k, v in acc.items()}
 
@@ -355,7 +356,6 @@ def bench_batched(torch, device, rank=0, world=1, max_over_ranks=lambda v: v, ba
     torch.cuda.synchronize()
     te = max_over_ranks(e0.elapsed_time(e1))
     st = batch.status()
-    passes = _batch_passes(scs)
     return {"value": total * n_sub / (tb * 1e-3), "unit": UNIT,
             "sequential_value": total * n_sub / (ts * 1e-3), "speedup_vs_sequential": ts / tb,
             "sequential_eager_value": total * n_sub / (te * 1e-3), "speedup_vs_sequential_eager": te / tb,
@@ -363,16 +363,11 @@ def bench_batched(torch, device, rank=0, world=1, max_over_ranks=lambda v: v, ba
             "scenes": len(all_scs), "particles": total, "grids": sorted({sc.n_grid for sc in all_scs}),
             "scenes_per_rank": len(scs), "substeps_per_frame": n_sub, "frames": reps,
             "tuned": {"knobs": tuned, "candidates_ms": autotune._CACHE[autotune.bucket(batch)]["ms"]},
-            "gpu_launches_per_substep": 7 + 3 * passes,
+            "gpu_launches_per_substep": LAUNCHES_PER_SUBSTEP,
             "nonfinite": sum(x["nonfinite"] for x in st),
             "what": "64 scenes, log-uniform 4k-256k particles, one BatchedAnisoMPM.run_frame per frame (one CUDA "
                     "graph) vs AnisoMPM.run_frame per scene (one CUDA graph each; and eager, one C call per "
                     "substep); scenes bin-packed across ranks"}
-
-
-def _batch_passes(scs):
-    from peel_mpm_b200 import _lib
-    return _lib.batch_workspace_layout([sc.n for sc in scs], [sc.n_grid for sc in scs]).ws.sort_passes
 
 
 def _smooth_field(torch, xs, gen, comps, modes=6):
@@ -759,7 +754,7 @@ def run_ours(args):
     floor_ms = (sum(NCU_KERNELS[k]["warp_inst"] for k in kern) / (4 * sm_count(torch) * clk * 1e6) * 1e3
                 if known else None)
     roof = {"bound": "hbm",
-            "kernel": " + ".join(kern) + (" (constitutive + P2G)" if dom == "p2g" else " (G2P)"),
+            "kernel": " + ".join(kern) + (" (binning + constitutive + P2G)" if dom == "p2g" else " (G2P)"),
             "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm, "peak_kind": peak_kind,
             "traffic": traffic, "traffic_over_algorithmic": (traffic / alg) if traffic else None,
             "algorithmic_bytes_per_launch": alg,
@@ -784,9 +779,6 @@ def run_ours(args):
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         cpu, parity = cpu_baseline(torch, device)
 
-    # clock, keys (+ first digit histogram), 3 per radix pass but the first's histogram, sub-block list,
-    # stress, tiles, compact, grid, g2p
-    launches_per_step = 7 + 3 * sim_passes(sim)
     if rank == 0:
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": ms_max / args.steps, "higher_is_better": True,
@@ -798,17 +790,12 @@ def run_ours(args):
                 "tuned": {"knobs": tuned, "candidates_ms": autotune._CACHE[autotune.bucket(sim)]["ms"],
                           "substeps_per_candidate": autotune._CACHE[autotune.bucket(sim)]["substeps"]},
                 "clocks": clocks.summary(), "roofline": roof, "cpu_baseline": cpu, "e2e": e2e,
-                "gpu_launches": launches_per_step * args.steps, "status": st, "late_run": late,
+                "gpu_launches": LAUNCHES_PER_SUBSTEP * args.steps, "status": st, "late_run": late,
                 "parity": parity}
         line.update(forms)
         print(json.dumps(line), flush=True)
     if world > 1:
         dist.destroy_process_group()
-
-
-def sim_passes(sim):
-    from peel_mpm_b200 import _lib
-    return _lib.workspace_layout(sim.n, sim.n_grid).sort_passes
 
 
 def main():

@@ -77,8 +77,7 @@ typedef struct pm_params {
     double f_clamp_hi;
     int32_t n_grips;
     int32_t n_colliders;
-    int32_t p2g_ctas_per_sm;    /* resident P2G CTAs per SM (0: the 80-register build, as many as fit;
-                                   4 or more: the 64-register build at 4 per SM; 1..3: a cap); a
+    int32_t p2g_ctas_per_sm;    /* cap on the resident P2G CTAs per SM (0: as many as fit, 3); a
                                    tuning knob with no effect on results (the grid sums are exact) */
     int32_t grid_ctas_per_sm;   /* grid-update CTAs per SM (0: the library default, else 1..64); a
                                    tuning knob with no effect on results */
@@ -146,8 +145,8 @@ size_t pm_struct_size(int32_t which);
  * graph, since attribute changes are not stream operations. */
 int pm_prepare(void);
 
-/* Workspace for n particles on an n_grid^3 grid: grids, sort buffers, block
- * lists and the control block.  Must be zeroed once by pm_workspace_init. */
+/* Workspace for n particles on an n_grid^3 grid: grids, sort buffers, cell
+ * table, P2G payload, block lists and the control block.  Must be zeroed once by pm_workspace_init. */
 int pm_workspace_size(int64_t n, int32_t n_grid, size_t *bytes);
 int pm_workspace_init(void *ws, size_t ws_bytes, int64_t n, int32_t n_grid, void *stream);
 
@@ -170,7 +169,7 @@ int pm_grid_sums(const void *ws, size_t ws_bytes, int64_t n, int32_t n_grid, flo
 
 /* ------------------------------------------------------------ the substep */
 
-/* Whole substep: clock, binning, P2G, grid update, G2P.
+/* Whole substep: clock, P2G (with its binning), grid update, G2P.
  * Replaces AnisoMPM.substep(time) (anisompm.py:593-803). */
 int pm_substep(const pm_params *prm, const pm_particles *P, void *ws, size_t ws_bytes,
                const pm_clock *clk, void *stream);
@@ -181,15 +180,17 @@ int pm_substep(const pm_params *prm, const pm_particles *P, void *ws, size_t ws_
 int pm_substep_dev_clock(const pm_params *prm, const pm_particles *P, void *ws, size_t ws_bytes,
                          const pm_clock *dev_clocks, int32_t row, void *stream);
 
-/* The pieces of pm_substep, in order.  Each needs the previous ones of the
- * same substep to have been enqueued. */
+/* The pieces of pm_substep, in order (pm_bin aside, which no other piece
+ * needs).  Each needs the previous ones of the same substep to have been
+ * enqueued. */
 int pm_set_clock(const pm_params *prm, void *ws, size_t ws_bytes, int64_t n, const pm_clock *clk,
                  void *stream);
-/* Binning of the substep: the quadratic base cell of every particle
- * (anisompm.py:544-548), numbered block-major (8^3-cell blocks, x-major;
- * a bijection of _node_index, anisompm.py:586-590), stable LSD radix sort of
- * (key, particle id), and the active 4^3 grid blocks.  No reference
- * counterpart: the reference scatters in particle order. */
+/* Sorts the particles by cell: the quadratic base cell of every particle
+ * (anisompm.py:544-548), numbered block-major (8^3-cell blocks, x-major, cells
+ * in Morton order; a bijection of _node_index, anisompm.py:586-590), stable LSD
+ * radix sort of (key, particle id).  pm_p2g does its own binning (a counting
+ * one) and does not need it.  No reference counterpart: the reference scatters
+ * in particle order. */
 int pm_bin(const pm_params *prm, const pm_particles *P, void *ws, size_t ws_bytes, void *stream);
 /* Particle BCs, constitutive update, damage update, degradation, quadratic
  * P2G and cubic damage scatter (anisompm.py:601-724, 768-776). */

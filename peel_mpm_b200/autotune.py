@@ -5,9 +5,8 @@ exact integers, every other kernel computes each particle or node the same
 way whatever its launch shape):
 
 * ``p2g_ctas_per_sm``: resident CTAs per SM of the persistent P2G kernel,
-  which takes 4^3-cell sub-blocks from a work list (0: the 80-register build
-  at 3 per SM; 4: the 64-register build at 4 per SM).  More CTAs hide more
-  latency; fewer registers spill a little.
+  which takes units of 4 x 4 x 8 cells from a work list: a cap (0, and any
+  value above 3: the 3 that fit).
 * ``stress_ctas_per_sm``: resident CTAs per SM of the constitutive update
   (3: the 80-register build; 4: the 64-register build, which spills a few
   values to L1 but runs more warps per SM).
@@ -31,7 +30,7 @@ from typing import Optional
 
 import torch
 
-P2G_CANDIDATES = (0, 2, 4)             # 0: as many as fit of the 80-register build (3 per SM)
+P2G_CANDIDATES = (0, 2, 4)             # 0: as many as fit (3 per SM)
 STRESS_CANDIDATES = (3, 4)
 G2P_CANDIDATES = (3, 4)
 GRID_CANDIDATES = (0, 4, 8, 16, 32)    # 0: one thread per node row

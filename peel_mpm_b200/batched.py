@@ -4,10 +4,10 @@
 objects into one device tensor (scene after scene) and re-points every
 scene's attribute views into it, so ``sims[k].x`` etc. keep working and show
 the batched results.  A substep of the batch runs the same kernels as
-``AnisoMPM.substep`` once over all scenes: one key pass, one radix sort of all
-scenes' keys (each scene owns a range of sort blocks), one P2G over sorted
-ranges (segments never cross scenes), one grid update over the active blocks
-of all grids and one G2P whose CTAs each belong to one scene.  Each scene
+``AnisoMPM.substep`` once over all scenes: one binning by counting in a table
+of all scenes' cells (each scene owns a range of it), one P2G over the
+non-empty units of cells (units never cross scenes), one grid update over the
+active blocks of all grids and one G2P whose CTAs each belong to one scene.  Each scene
 keeps its own grid size, dx, dt, parameters, grips, colliders, clock and step
 counter.  ``run_frame`` captures the frame in a CUDA graph whose per-scene
 times come from a device table, as ``AnisoMPM.run_frame`` does.

@@ -10,13 +10,13 @@
 // adjoint then runs four kernels:
 //   k_adj_pre       per particle (particle order): the G2P tail adjoint and
 //                   the G2P adjoint's scatter payload, written to the
-//                   particle's slot of the forward substep's recorded sort,
+//                   particle's recorded place of the forward substep,
 //                   and the bounds that fix the fixed-point units;
-//   k_adj_tiles     G2P adjoint as a scatter over the recorded sub-block work
-//                   list (the forward P2G's cell-aggregated tiles): the adjoint
-//                   of the grid velocity and damage field in int64 fixed
-//                   point, so the sums do not depend on the atomics' order and
-//                   a backward pass is reproducible bit for bit;
+//   k_adj_sweep     G2P adjoint as a scatter over the recorded unit list (the
+//                   forward P2G's sweep): the adjoint of the grid velocity and
+//                   damage field in int64 fixed point, so the sums do not
+//                   depend on the atomics' order and a backward pass is
+//                   reproducible bit for bit;
 //   k_adj_grid      grid-update adjoint over the recorded active blocks
 //                   (normalisation by mass and by the cubic weight sum);
 //   k_adj_particle  P2G adjoint as a gather plus the constitutive adjoint
@@ -30,6 +30,7 @@
 // recorded pre-collider grid velocity (resolve_adj), and the directional
 // stress at interface particles by dir_adjoint.
 #include "pm_kernels.cuh"
+#include "pm_sweep.cuh"
 
 namespace pm {
 
@@ -43,7 +44,7 @@ struct TapeHead {
     int any_allow;
     long long step;
     double time;
-    unsigned n_work;    // non-empty sub-blocks of the substep's sort
+    unsigned n_work;    // non-empty units of the substep
     unsigned pad;
     float col_origin[PM_MAX_COLLIDERS][3];   // the substep's collider origins and velocities
     float col_vel[PM_MAX_COLLIDERS][3];
@@ -53,7 +54,7 @@ struct TapeHead {
 // contributions (float bits) and the dynamic work cursor.
 struct AdjCtrl {
     unsigned mom_bound, lap_bound, work_next, pad;
-    unsigned slots[2][kBoundSlots];   // per-warp-slot bounds, folded by k_adj_bounds
+    unsigned slots[2][kBoundSlots];   // per-warp-slot bounds, folded by k_adj_sweep
 };
 
 // Quadratic weights with their derivatives wrt the local coordinate fx.
@@ -173,13 +174,10 @@ __device__ __forceinline__ void g2p_input_F(const pm_params &prm, const float *_
 // Adjoint of v' = sum w v_i, C' = K sum w v_i dpos^T and lap' = sum L gd_i has
 // the form of a P2G scatter: node i receives w (vt + K Ct dpos) and
 // lb (w''x wy wz + wx w''y wz + wx wy w''z) with lb = L lapbar.  This kernel
-// forms each particle's {fx | x, lb}, vt and K Ct (the momentum scatter's
-// {fx, mv, aff} slots) at its position in the forward substep's sort.
-constexpr int kAdjCW = 30;   // expanded cubic w and w'' per particle (5 per axis each)
-
+// forms each particle's payload {fx | x, lb}, {vt, 0}, K Ct at its recorded place.
 __global__ void __launch_bounds__(256) k_adj_pre(const pm_params prm, const Parts pre, const Parts post,
                                                  const pm_state_adj ain, const int *__restrict__ iperm,
-                                                 float4 *__restrict__ pay, AdjCtrl *actl,
+                                                 void *__restrict__ pay, AdjCtrl *actl,
                                                  const float *__restrict__ tpol, long long rs) {
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= pre.n) return;
@@ -215,12 +213,15 @@ __global__ void __launch_bounds__(256) k_adj_pre(const pm_params prm, const Part
         reg = reg && (fb >= 1.0f) && (fb <= (float)(ng - 4));
         fx[ax] = __fsub_rn(X, fb);
     }
-    float4 *dst = pay + 5 * (long long)iperm[p];
-    dst[0] = reg ? make_float4(fx[0], fx[1], fx[2], 0.0f) : make_float4(xp[0], xp[1], xp[2], 0.0f);
-    dst[1] = make_float4(vt[0], vt[1], vt[2], lb);
-    dst[2] = make_float4(kc[0], kc[1], kc[2], kc[3]);
-    dst[3] = make_float4(kc[4], kc[5], kc[6], kc[7]);
-    dst[4] = make_float4(kc[8], reg ? 1.0f : 0.0f, 0.0f, 0.0f);
+    {
+        const long long at = iperm[p];
+        float4 *dst = (float4 *)pay_at(pay, at);
+        dst[0] = reg ? make_float4(fx[0], fx[1], fx[2], lb) : make_float4(xp[0], xp[1], xp[2], lb);
+        dst[32] = make_float4(vt[0], vt[1], vt[2], 0.0f);
+        dst[64] = make_float4(kc[0], kc[3], kc[1], kc[4]);
+        dst[96] = make_float4(kc[2], kc[5], kc[6], kc[7]);
+        *pay_az2(pay, at) = kc[8];
+    }
     // bounds of one node contribution: |w (vt + K Ct dpos)| with w <= 1,
     // |dpos| <= 1.5 dx per axis (the cubic stencil's quadratic part), and
     // |lb W''| with |w''x wy wz + wx w''y wz + wx wy w''z| <= 3 (|w''| <= 2, w <= 2/3)
@@ -237,24 +238,6 @@ __global__ void __launch_bounds__(256) k_adj_pre(const pm_params prm, const Part
         const int slot = (int)(((blockIdx.x << 3) + (threadIdx.x >> 5)) & (kBoundSlots - 1));
         atomicMax(&actl->slots[0][slot], bmom);
         atomicMax(&actl->slots[1][slot], blap);
-    }
-}
-
-__global__ void __launch_bounds__(kBoundSlots) k_adj_bounds(AdjCtrl *actl) {
-    __shared__ unsigned s_m[2][kBoundSlots / 32];
-    const int t = threadIdx.x;
-#pragma unroll
-    for (int v = 0; v < 2; ++v) {
-        const unsigned m = __reduce_max_sync(0xffffffffu, actl->slots[v][t]);
-        if ((t & 31) == 0) s_m[v][t >> 5] = m;
-    }
-    __syncthreads();
-    if (t < 2) {
-        unsigned m = 0u;
-#pragma unroll
-        for (int k = 0; k < kBoundSlots / 32; ++k) m = max(m, s_m[t][k]);
-        if (t == 0) actl->mom_bound = m;
-        else actl->lap_bound = m;
     }
 }
 
@@ -309,291 +292,97 @@ __device__ __noinline__ void adj_scatter_global(const float xp[3], const float v
         }
 }
 
-// ---------------------------------------------------------------- k_adj_tiles
-// The G2P adjoint scatter over the forward substep's non-empty 4^3-cell
-// sub-blocks, with the forward P2G's cell-aggregated (cell, x-slab) items:
-// quadratic slabs sum w (vt + K Ct dpos) into the momentum-adjoint tile
-// (nodes [4s, 4s+6)^3), cubic slabs sum lb W'' into the damage-adjoint tile
-// (nodes [4s-1, 4s+7)^3), both int64 fixed point, flushed with one atomic per
-// touched node and component.  The adjoint touches exactly the nodes the
-// forward P2G touched, so no block marks are needed.
-constexpr int kATh = 256;
-constexpr int kAPayStride = kATh + kATh / 32;
-constexpr int kASub = 4, kAQE = 6, kACE = 8, kAQN = 216, kACN = 512;
-// chunk planes with the forward P2G's conflict-free strides (z 1, y 8, x 52 / 68)
-constexpr int kAQSY = 8, kAQSX = 52, kAQPl = 312, kACSY = 8, kACSX = 68, kACPl = 544;
-constexpr size_t kAdjTileSmem = sizeof(unsigned) * 2 * (3 * kAQPl + kACPl) +
-                                sizeof(float) * (17 + kAdjCW) * kAPayStride + sizeof(int) * (kATh + 2) + 2 * kATh;
-
-__global__ void __launch_bounds__(kATh, 3) k_adj_tiles(const pm_params prm, const unsigned *__restrict__ keys,
-                                                       const int *__restrict__ work, const TapeHead *head,
-                                                       const float4 *__restrict__ pay, AdjCtrl *actl,
-                                                       long long *__restrict__ acc, long long n) {
-    extern __shared__ long long s_adj[];
-    unsigned (*qlo)[kAQPl] = (unsigned (*)[kAQPl])(s_adj);                // [3][kAQPl] chunk planes
-    int (*qhi)[kAQPl] = (int (*)[kAQPl])(qlo[3]);                         // [3][kAQPl]
-    unsigned *clo = (unsigned *)(qhi[3]);                                 // [kACPl]
-    int *chi = (int *)(clo + kACPl);                                      // [kACPl]
-    float (*sp)[kAPayStride] = (float (*)[kAPayStride])(chi + kACPl);    // [17][kAPayStride]
-    float (*cw)[kAPayStride] = (float (*)[kAPayStride])(sp[17]);        // [kAdjCW][kAPayStride]
-    int *runs = (int *)(cw[kAdjCW]);                                      // [kATh + 2]
-    unsigned char *regular = (unsigned char *)(runs + kATh + 2);          // [kATh]
-    unsigned char *lcell = regular + kATh;                                // [kATh]
-    __shared__ int s_wcnt[kATh / 32];
-    __shared__ unsigned s_item;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const unsigned n_work = min(head->n_work, (unsigned)min(n, (long long)0x7fffffff));
-    const int ng = prm.n_grid;
-    const int nb = sort_blocks_per_axis(ng);
-    const float inv_dx = (float)prm.inv_dx, dx = (float)prm.dx;
-    const float smom = fix_scale(actl->mom_bound).scale, slap = fix_scale(actl->lap_bound).scale;
-    for (int i = tid; i < 2 * (3 * kAQPl + kACPl); i += kATh) qlo[0][i] = 0u;
-    for (;;) {
-        __syncthreads();
-        if (tid == 0) s_item = atomicAdd(&actl->work_next, 1u);
-        __syncthreads();
-        const unsigned item = s_item;
-        if (item >= n_work) break;
-        const long long a = work[item];
-        const unsigned key0 = keys[a];
-        const unsigned sbk = key0 >> 6;
-        const unsigned blk = key0 >> kSortBlockBits;
-        const int bz = (int)(blk % nb), by = (int)((blk / nb) % nb), bx = (int)(blk / ((unsigned)nb * nb));
-        const unsigned oct = (key0 >> 6) & 7u;
-        const int org[3] = {bx * kSortBlock + (int)((oct >> 2) & 1u) * kASub,
-                            by * kSortBlock + (int)((oct >> 1) & 1u) * kASub,
-                            bz * kSortBlock + (int)(oct & 1u) * kASub};
-        int pending = 0;   // chunks with particles since the planes were last folded
-        for (long long sub = a;; sub += kATh) {
-            const long long i = sub + tid;
-            const unsigned key = i < n ? keys[i] : 0xffffffffu;
-            const bool valid = i < n && (key >> 6) == sbk;
-            if (valid) {
-                const float4 *src = pay + 5 * i;
-                const float4 q0 = src[0], q1 = src[1], q2 = src[2], q3 = src[3], q4 = src[4];
-                const int t = tid + (tid >> 5);
-                sp[0][t] = q0.x; sp[1][t] = q0.y; sp[2][t] = q0.z;
-                sp[3][t] = q1.x; sp[4][t] = q1.y; sp[5][t] = q1.z; sp[16][t] = q1.w;
-                sp[6][t] = q2.x; sp[7][t] = q2.y; sp[8][t] = q2.z; sp[9][t] = q2.w;
-                sp[10][t] = q3.x; sp[11][t] = q3.y; sp[12][t] = q3.z; sp[13][t] = q3.w;
-                sp[14][t] = q4.x;
-                regular[tid] = q4.y != 0.0f ? 1 : 0;
-                lcell[tid] = (unsigned char)(key & 63u);
-                if (q4.y != 0.0f) {
-                    float e[5];
-                    cw5(q0.x, e);
+// ---------------------------------------------------------------- k_adj_sweep
+// The G2P adjoint scatter over the forward substep's non-empty units, with the
+// forward P2G's sweep (pm_sweep.cuh): quadratic planes sum w (vt + K Ct dpos)
+// into the momentum adjoint, cubic planes lb W'' into the damage adjoint, int64
+// fixed point.  The adjoint touches exactly the nodes the forward P2G touched,
+// so no block marks are needed.
+__global__ void __launch_bounds__(kSweepThreads, 3) k_adj_sweep(const __grid_constant__ pm_params prm,
+                                                                const int *__restrict__ work,
+                                                                const int2 *__restrict__ cells,
+                                                                const unsigned char *__restrict__ split,
+                                                                const TapeHead *head,
+                                                                void *pay, AdjCtrl *actl, long long *__restrict__ acc,
+                                                                long long n) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    SweepShared &sh = *(SweepShared *)s_raw;
+    int tid;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
+    const int lane = tid & 31, wid = __reduce_max_sync(0xffffffffu, tid >> 5);
+    const unsigned n_units = min(head->n_work, (unsigned)min(n, (long long)0x1fffffff));
+    const int parts = sweep_parts(n_units), layers = kUnitX / parts;
+    const unsigned n_work = n_units * parts;   // an item is a unit's layers part * layers .. + layers
+    const int ng = prm.n_grid, nb = sort_blocks_per_axis(ng);
+    for (int i = tid; i < kSweepQ * 4 * kQRows * kPlaneCols; i += kSweepThreads) sh.qpl[0][0][i] = 0;
+    for (int i = tid; i < kSweepC * 2 * kCRows * kPlaneCols; i += kSweepThreads) sh.cpl[0][0][i] = 0;
+    if (wid >= 4 && wid < 6) {            // fold the bound slots (kept for the grid adjoint too)
+        unsigned m = 0;
 #pragma unroll
-                    for (int k = 0; k < 5; ++k) cw[k][t] = e[k];
-                    cw5(q0.y, e);
-#pragma unroll
-                    for (int k = 0; k < 5; ++k) cw[5 + k][t] = e[k];
-                    cw5(q0.z, e);
-#pragma unroll
-                    for (int k = 0; k < 5; ++k) cw[10 + k][t] = e[k];
-                    cw5_2(q0.x, e);
-#pragma unroll
-                    for (int k = 0; k < 5; ++k) cw[15 + k][t] = e[k];
-                    cw5_2(q0.y, e);
-#pragma unroll
-                    for (int k = 0; k < 5; ++k) cw[20 + k][t] = e[k];
-                    cw5_2(q0.z, e);
-#pragma unroll
-                    for (int k = 0; k < 5; ++k) cw[25 + k][t] = e[k];
-                }
-            }
-            int nruns, cnt;
-            {
-                const unsigned prev = (tid > 0 && i <= n) ? keys[i - 1] : 0xffffffffu;
-                const bool flag = valid && (tid == 0 || key != prev);
-                const unsigned fb = __ballot_sync(0xffffffffu, flag), vb = __ballot_sync(0xffffffffu, valid);
-                if (lane == 0) s_wcnt[wid] = (int)(__popc(fb) | (__popc(vb) << 16));
-                __syncthreads();
-                int pos = __popc(fb & lanemask_lt()), tot = 0, vt = 0;
-#pragma unroll
-                for (int w2 = 0; w2 < kATh / 32; ++w2) {
-                    const int c = s_wcnt[w2];
-                    pos += (w2 < wid) ? (c & 0xffff) : 0;
-                    tot += c & 0xffff;
-                    vt += c >> 16;
-                }
-                if (flag) runs[pos] = tid;
-                if (tid == 0) runs[tot] = vt;
-                nruns = tot;
-                cnt = vt;
-                __syncthreads();
-            }
-            if (valid && !regular[tid]) {
-                const int t = tid + (tid >> 5);
-                const float xp[3] = {sp[0][t], sp[1][t], sp[2][t]};
-                const float vt[3] = {sp[3][t], sp[4][t], sp[5][t]};
-                float kc[9];
-#pragma unroll
-                for (int k = 0; k < 9; ++k) kc[k] = sp[6 + k][t];
-                adj_scatter_global(xp, vt, kc, sp[16][t], inv_dx, dx, ng, smom, slap, acc);
-            }
-            for (int it = tid; it < nruns * 8; it += kATh) {   // slab-major, as the forward P2G
-                const bool quad = it < 3 * nruns;
-                const int k = quad ? it : it - 3 * nruns;
-                const int s8 = k / nruns;
-                const int r = k - s8 * nruns;
-                const int sl = quad ? s8 : 3 + s8;
-                const int ja = runs[r], jb = runs[r + 1];
-                int cq[3];
-                morton_decode(lcell[ja], cq);
-                if (sl < 3) {
-                    const int ox = sl;
-                    // packed pairs: components (0, 1) of every node, component 2 alone
-                    float2 acc01[3][3];
-                    float acc2[3][3];
-#pragma unroll
-                    for (int i2 = 0; i2 < 3; ++i2)
-#pragma unroll
-                        for (int j = 0; j < 3; ++j) {
-                            acc01[i2][j] = make_float2(0.0f, 0.0f);
-                            acc2[i2][j] = 0.0f;
-                        }
-                    // a cell's particles share their base cell: all regular or all not
-                    const int jend = regular[ja] ? jb : ja;
-                    for (int j = ja; j < jend; ++j) {
-                        const int t = j + (j >> 5);
-                        const float fx0 = sp[0][t], fx1 = sp[1][t], fx2 = sp[2][t];
-                        float wx[3], wy[3], wz[3];
-                        qw(fx0, wx); qw(fx1, wy); qw(fx2, wz);
-                        const float dxo = ((float)ox - fx0) * dx;
-                        const float2 base01 = fma2(make_float2(sp[6][t], sp[9][t]), bc2(dxo),
-                                                   make_float2(sp[3][t], sp[4][t]));
-                        const float base2 = sp[5][t] + sp[12][t] * dxo;
-                        const float2 ay01 = make_float2(sp[7][t], sp[10][t]), az01 = make_float2(sp[8][t], sp[11][t]);
-                        const float ay2 = sp[13][t], az2 = sp[14][t];
-                        const float wxs = ox == 0 ? wx[0] : (ox == 1 ? wx[1] : wx[2]);
-                        // w (base + a_y dy + a_z dz) = wxy [wz (base + a_z dz)] + [wxy a_y dy] wz
-                        float2 bz01[3], wz2[3];
-                        float bz2[3];
-#pragma unroll
-                        for (int oz = 0; oz < 3; ++oz) {
-                            const float dz = ((float)oz - fx2) * dx;
-                            wz2[oz] = bc2(wz[oz]);
-                            bz01[oz] = mul2(wz2[oz], fma2(az01, bc2(dz), base01));
-                            bz2[oz] = wz[oz] * (base2 + az2 * dz);
-                        }
-#pragma unroll
-                        for (int oy = 0; oy < 3; ++oy) {
-                            const float wxy = wxs * wy[oy];
-                            const float wdy = wxy * (((float)oy - fx1) * dx);
-                            const float2 w2 = bc2(wxy), ady01 = mul2(bc2(wdy), ay01);
-                            const float ady2 = wdy * ay2;
-#pragma unroll
-                            for (int oz = 0; oz < 3; ++oz) {
-                                acc01[oy][oz] = fma2(ady01, wz2[oz], fma2(w2, bz01[oz], acc01[oy][oz]));
-                                acc2[oy][oz] = fmaf(ady2, wz[oz], fmaf(wxy, bz2[oz], acc2[oy][oz]));
-                            }
-                        }
-                    }
-                    const int nx = cq[0] + ox;
-#pragma unroll
-                    for (int oy = 0; oy < 3; ++oy)
-#pragma unroll
-                        for (int oz = 0; oz < 3; ++oz) {
-                            const int sidx = nx * kAQSX + (cq[1] + oy) * kAQSY + cq[2] + oz;
-                            plane_add(&qlo[0][sidx], &qhi[0][sidx], acc01[oy][oz].x, smom);
-                            plane_add(&qlo[1][sidx], &qhi[1][sidx], acc01[oy][oz].y, smom);
-                            plane_add(&qlo[2][sidx], &qhi[2][sidx], acc2[oy][oz], smom);
-                        }
-                } else {
-                    const int nxs = sl - 3;
-                    // packed pairs of z-neighbours: nodes (0, 1), (2, 3) of a row, node 4 alone
-                    float2 al01[5], al23[5];
-                    float al4[5];
-#pragma unroll
-                    for (int i2 = 0; i2 < 5; ++i2) {
-                        al01[i2] = al23[i2] = make_float2(0.0f, 0.0f);
-                        al4[i2] = 0.0f;
-                    }
-                    const int jend = regular[ja] ? jb : ja;
-                    for (int j = ja; j < jend; ++j) {
-                        const int t = j + (j >> 5);
-                        const float lb = sp[16][t];
-                        const float ax = lb * cw[15 + nxs][t], bx2 = lb * cw[nxs][t];   // lb w''x, lb wx
-                        const float2 ez01 = make_float2(cw[10][t], cw[11][t]), ez23 = make_float2(cw[12][t], cw[13][t]);
-                        const float2 e2z01 = make_float2(cw[25][t], cw[26][t]), e2z23 = make_float2(cw[27][t], cw[28][t]);
-                        const float ez4 = cw[14][t], e2z4 = cw[29][t];
-#pragma unroll
-                        for (int ny = 0; ny < 5; ++ny) {
-                            const float wy = cw[5 + ny][t], w2y = cw[20 + ny][t];
-                            const float t1 = ax * wy + bx2 * w2y;   // (w''x wy + wx w''y) lb
-                            const float t2 = bx2 * wy;              // wx wy lb
-                            const float2 t12 = bc2(t1), t22 = bc2(t2);
-                            al01[ny] = fma2(t22, e2z01, fma2(t12, ez01, al01[ny]));
-                            al23[ny] = fma2(t22, e2z23, fma2(t12, ez23, al23[ny]));
-                            al4[ny] = fmaf(t2, e2z4, fmaf(t1, ez4, al4[ny]));
-                        }
-                    }
-                    const int nx = cq[0] + nxs;
-#pragma unroll
-                    for (int ny = 0; ny < 5; ++ny)
-#pragma unroll
-                        for (int nz = 0; nz < 5; ++nz)
-                        {
-                            const int sidx = nx * kACSX + (cq[1] + ny) * kACSY + cq[2] + nz;
-                            const float a = nz == 0 ? al01[ny].x : nz == 1 ? al01[ny].y : nz == 2 ? al23[ny].x
-                                          : nz == 3 ? al23[ny].y : al4[ny];
-                            plane_add(&clo[sidx], &chi[sidx], a, slap);
-                        }
-                }
-            }
-            __syncthreads();
-            const bool last = cnt < kATh;
-            pending += cnt > 0 ? 1 : 0;
-            // fold the chunk planes straight into the global grid, one int64
-            // atomic per nonzero node component, after every second chunk with
-            // particles and after the last: one add per particle and node is
-            // below 0.89 of 2^46 units (|w''x wy wz + wx w''y wz + wx wy w''z|
-            // <= 2.67 against the bound's 3), so two chunks keep the high
-            // plane under 512 * 0.89 * 2^22 < 2^31
-            if (pending > 0 && (last || pending == 2)) {
-                pending = 0;
-                for (int li = tid; li < kAQN; li += kATh) {
-                    const int tx = li / (kAQE * kAQE), ty = (li / kAQE) % kAQE, tz = li % kAQE;
-                    const int sidx = tx * kAQSX + ty * kAQSY + tz;
-                    long long q[3];
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        const unsigned lo = qlo[c][sidx];
-                        const int hi = qhi[c][sidx];
-                        q[c] = 0;
-                        if ((lo | (unsigned)hi) != 0u) {
-                            qlo[c][sidx] = 0u;
-                            qhi[c][sidx] = 0;
-                            q[c] = plane_value(lo, hi);
-                        }
-                    }
-                    if ((q[0] | q[1] | q[2]) != 0) {
-                        long long *g = acc + 4 * (((long long)(org[0] + tx) * ng + (org[1] + ty)) * ng + (org[2] + tz));
-#pragma unroll
-                        for (int c = 0; c < 3; ++c)
-                            if (q[c]) atomicAdd((unsigned long long *)(g + c), (unsigned long long)q[c]);
-                    }
-                }
-                for (int li = tid; li < kACN; li += kATh) {
-                    const int tx = li >> 6, ty = (li >> 3) & 7, tz = li & 7;
-                    const int sidx = tx * kACSX + ty * kACSY + tz;
-                    const unsigned lo = clo[sidx];
-                    const int hi = chi[sidx];
-                    if ((lo | (unsigned)hi) != 0u) {
-                        clo[sidx] = 0u;
-                        chi[sidx] = 0;
-                        const long long q3 = plane_value(lo, hi);
-                        if (q3 != 0) {
-                            long long *g = acc + 4 * (((long long)(org[0] - 1 + tx) * ng + (org[1] - 1 + ty)) * ng +
-                                                      (org[2] - 1 + tz));
-                            atomicAdd((unsigned long long *)(g + 3), (unsigned long long)q3);
-                        }
-                    }
-                }
-            }
-            if (last) break;
-            __syncthreads();
+        for (int k = 0; k < kBoundSlots / 32; ++k) m = max(m, actl->slots[wid - 4][k * 32 + lane]);
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (lane == 0) {
+            sh.scale[2 * (wid - 4)] = fix_scale(m).scale;
+            if (wid == 4) actl->mom_bound = m;
+            else actl->lap_bound = m;
         }
+    }
+    if (tid == 0) sh.next.x = (int)atomicAdd(&actl->work_next, 1u);
+    __syncthreads();
+    unsigned item = (unsigned)sh.next.x;
+    while (item < n_work) {
+        const unsigned i = item / parts;   // place in the list
+        const int u = work[i], x0 = (int)(item - i * parts) * layers, x1 = x0 + layers;
+        const unsigned blk = (unsigned)u / kBlockUnits;
+        const int org[3] = {(int)(blk / ((unsigned)nb * nb)) * kSortBlock + ((u >> 1) & 1) * kUnitX,
+                            (int)(blk / nb % nb) * kSortBlock + (u & 1) * kUnitY, (int)(blk % nb) * kSortBlock};
+        bool edge = false;                // particles that need clamped nodes
+        int2 cell = make_int2(0, 0);
+        if (wid >= x0 && wid < x1) {
+            cell = cells[(long long)i * kUnitCells + tid];
+            const int c[3] = {tid >> 5, (tid >> 3) & 3, tid & 7};
+            bool reg = true;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) reg = reg && org[a] + c[a] >= 1 && org[a] + c[a] <= ng - 4;
+            edge = cell.y > 0 && !reg;
+            const int cnt = reg ? cell.y : 0;
+            sh.cell[tid] = make_int2(cell.x, cnt);
+            sh.split[tid] = split[(long long)i * kUnitCells + tid];
+            const int rows = __reduce_max_sync(0xffffffffu, cnt);
+            if (lane == 0) sh.layer_rows[wid] = rows;
+        }
+        if (tid == kSweepThreads - 1) {
+            sh.ng = ng;
+            sh.dx = (float)prm.dx;
+            sh.g_quad = acc + 4 * (((long long)org[0] * ng + org[1]) * ng + org[2]);
+            sh.g_cubic = acc + 4 * (((long long)(org[0] - 1) * ng + org[1] - 1) * ng + org[2] - 1) + 3;
+        }
+        const bool edges = __syncthreads_or(edge);
+        unsigned take = 0;                // the next item is taken while this one is swept
+        if (tid == kSweepThreads - 1) take = atomicAdd(&actl->work_next, 1u);
+        if (edges) {                      // the cell's particles over the lanes of its warp
+            const unsigned eb = __ballot_sync(0xffffffffu, edge);
+            for (unsigned m = eb; m; m &= m - 1) {
+                const int l = __ffs(m) - 1;
+                const int f = __shfl_sync(0xffffffffu, cell.x, l), cnt = __shfl_sync(0xffffffffu, cell.y, l);
+                for (int k = lane; k < cnt; k += 32) {
+                    const long long s = place_of(f, k);
+                    const float4 *p = (const float4 *)pay_at(pay, s);
+                    const float4 p0 = p[0], p1 = p[32], p2 = p[64], p3 = p[96];
+                    const float xp[3] = {p0.x, p0.y, p0.z}, vt[3] = {p1.x, p1.y, p1.z};
+                    const float kc[9] = {p2.x, p2.z, p3.x, p2.y, p2.w, p3.y, p3.z, p3.w, *pay_az2(pay, s)};
+                    adj_scatter_global(xp, vt, kc, p0.w, (float)prm.inv_dx, (float)prm.dx, ng, sh.scale[0], sh.scale[2], acc);
+                }
+            }
+        }
+        if (wid < kSweepQ)
+            sweep_warp<QuadSums<true>, kSweepQ>(sh, sh.qring[wid], (const char *)pay, wid, wid, lane, x0, x1);
+        else
+            sweep_warp<CubicLapSums, kSweepC>(sh, sh.cring[wid - kSweepQ], (const char *)pay, wid, wid - kSweepQ, lane, x0,
+                                             x1);
+        if (tid == kSweepThreads - 1) sh.next.x = (int)take;
+        __syncthreads();
+        item = (unsigned)sh.next.x;
     }
 }
 
@@ -1595,7 +1384,7 @@ void prepare_adjoint() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(k_adj_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAdjTileSmem);
+        cudaFuncSetAttribute(k_adj_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SweepShared));
         done[dev] = 1;
     }
 }
@@ -1607,6 +1396,8 @@ TapeLayout make_tape_layout(long long n, int ng, int slots, int flags) {
     const long long G = (long long)ng * ng * ng;
     const int nbs = (ng + kBlockEdge - 1) / kBlockEdge;
     const long long nb = (long long)nbs * nbs * nbs;
+    const long long nb8 = sort_blocks_per_axis(ng);
+    const long long units = std::max<long long>(1, std::min(n, nb8 * nb8 * nb8 * kBlockUnits));   // listed at most
     const long long np = (n + 63) / 64 * 64 > 0 ? (n + 63) / 64 * 64 : 64;
     size_t o = 0;
     T.head = o;    o = align_up(o + sizeof(TapeHead) * (size_t)(slots > 0 ? slots : 1), A);
@@ -1614,7 +1405,7 @@ TapeLayout make_tape_layout(long long n, int ng, int slots, int flags) {
     T.acc = o;     o = align_up(o + 32 * (size_t)G, A);     // 4 x int64 per node
     T.adj_q = o;   o = align_up(o + 16 * (size_t)G, A);
     T.adj_c = o;   o = align_up(o + 16 * (size_t)G, A);
-    T.apay = o;    o = align_up(o + 80 * (size_t)np, A);
+    T.apay = o;    o = align_up(o + kPayBytes * (size_t)(kPayPlaces * np), A);   // (np is a multiple of 32)
     T.slot0 = o;
     size_t s = 0;
     T.vel = s;     s = align_up(s + 16 * (size_t)G, A);
@@ -1622,9 +1413,10 @@ TapeLayout make_tape_layout(long long n, int ng, int slots, int flags) {
     T.sw = s;      s = align_up(s + 4 * (size_t)G, A);
     T.vpre = s;    s = align_up(s + ((flags & PM_TAPE_COLLIDERS) ? 16 * (size_t)G : 0), A);   // pre-collider v
     T.blocks = s;  s = align_up(s + 4 * (size_t)nb, A);
-    T.keys = s;    s = align_up(s + 4 * (size_t)np, A);
     T.iperm = s;   s = align_up(s + 4 * (size_t)np, A);
     T.work = s;    s = align_up(s + 4 * (size_t)np, A);
+    T.split = s;   s = align_up(s + (size_t)kUnitCells * (size_t)units, A);
+    T.cells = s;   s = align_up(s + 8 * (size_t)kUnitCells * (size_t)units, A);
     T.aff = s;     s = align_up(s + 36 * (size_t)np, A);
     T.pol = s;     s = align_up(s + 88 * (size_t)np, A);
     T.aff_stride = np;
@@ -1643,20 +1435,17 @@ void record_redirect(const TapeLayout &T, void *tape, int slot, WS &w) {
     w.g_sw = (float *)(b + T.sw);
     w.g_vpre = (T.flags & PM_TAPE_COLLIDERS) ? (float4 *)(b + T.vpre) : nullptr;
     w.block_list = (int *)(b + T.blocks);
-    w.inv_perm = (int *)(b + T.iperm);   // the substep's sort stays on the tape for the adjoint
+    w.slot = (int *)(b + T.iperm);       // the particles' places, the unit list and its cells stay on the tape
     w.work = (int *)(b + T.work);
+    w.rec_cells = (int2 *)(b + T.cells);
+    w.rec_split = (unsigned char *)(b + T.split);
     w.tape_aff = (float *)(b + T.aff);
     w.tape_pol = (float *)(b + T.pol);
     w.tape_aff_stride = T.aff_stride;
 }
 
 void launch_tape_head(const TapeLayout &T, void *tape, int slot, const WS &w, long long n, cudaStream_t s) {
-    TapeHead *h = (TapeHead *)((char *)tape + T.head) + slot;
-    k_tape_head<<<1, 32, 0, s>>>(w.ctrl, h, n);
-    if (n > 0) {
-        char *b = (char *)tape + T.slot0 + T.slot_bytes * (size_t)slot;
-        cudaMemcpyAsync(b + T.keys, w.sorted_keys, 4 * (size_t)n, cudaMemcpyDeviceToDevice, s);
-    }
+    k_tape_head<<<1, 32, 0, s>>>(w.ctrl, (TapeHead *)((char *)tape + T.head) + slot, n);
 }
 
 void launch_adjoint(const pm_params &prm, const Parts &pre, const Parts &post, const pm_state_adj &ain,
@@ -1667,7 +1456,7 @@ void launch_adjoint(const pm_params &prm, const Parts &pre, const Parts &post, c
     const TapeHead *h = (const TapeHead *)(base + T.head) + slot;
     AdjCtrl *actl = (AdjCtrl *)(base + T.actl);
     long long *acc = (long long *)(base + T.acc);
-    float4 *apay = (float4 *)(base + T.apay);
+    void *apay = base + T.apay;
     float4 *Aq = (float4 *)(base + T.adj_q);
     float4 *Bc = (float4 *)(base + T.adj_c);
     const float4 *gvel = (const float4 *)(b + T.vel);
@@ -1680,19 +1469,18 @@ void launch_adjoint(const pm_params &prm, const Parts &pre, const Parts &post, c
     cudaMemsetAsync(actl, 0, sizeof(AdjCtrl), s);
     k_adj_pre<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(prm, pre, post, ain, (const int *)(b + T.iperm), apay, actl,
                                                           (const float *)(b + T.pol), T.aff_stride);
-    k_adj_bounds<<<1, kBoundSlots, 0, s>>>(actl);
     {
         static int slots_dev[64] = {0};
         int dev = 0;
         cudaGetDevice(&dev);
         int slots = (dev >= 0 && dev < 64) ? slots_dev[dev] : 0;
         if (slots <= 0) {
-            slots = resident_slots((const void *)k_adj_tiles, kATh, kAdjTileSmem);
+            slots = resident_slots((const void *)k_adj_sweep, kSweepThreads, sizeof(SweepShared));
             if (dev >= 0 && dev < 64) slots_dev[dev] = slots;
         }
-        const long long blocks_t = std::max<long long>(1, std::min<long long>(slots, (n + 63) / 64));
-        k_adj_tiles<<<(unsigned)blocks_t, kATh, kAdjTileSmem, s>>>(prm, (const unsigned *)(b + T.keys),
-                                                                  (const int *)(b + T.work), h, apay, actl, acc, n);
+        k_adj_sweep<<<(unsigned)std::min<long long>(slots, n), kSweepThreads, sizeof(SweepShared), s>>>(
+            prm, (const int *)(b + T.work), (const int2 *)(b + T.cells), (const unsigned char *)(b + T.split), h,
+            apay, actl, acc, n);
     }
     const long long max_items = T.n_blocks * 64;
     const int gb = (int)std::max<long long>(1, std::min<long long>((max_items + 255) / 256, 148LL * 8));

@@ -1,11 +1,11 @@
 // Batched substep: many independent scenes, packed into one particle array,
-// advanced by one launch per kernel over the work of all scenes (one key
-// pass, one radix sort, one P2G, one grid update, one G2P).
+// advanced by one launch per kernel over the work of all scenes (one binning
+// pass, one P2G, one grid update, one G2P).
 //
 // Packing: scene s owns particles [pb[s], pb[s+1]) of the concatenated planes,
 // grid nodes [nodeb[s], nodeb[s] + ng_s^3) of one node buffer, sort blocks
 // [sblk[s], sblk[s+1]) of one key space, 4^3 grid blocks [gblk[s], gblk[s+1])
-// of one block mask and G2P CTAs [ctab[s], ctab[s+1]).  The scene tables and
+// of one block mask and 256-particle CTAs [ctab[s], ctab[s+1]).  The scene tables and
 // the per-scene parameters live in the workspace, so a captured graph of
 // pm_batch_substep calls needs no host data; the host derives launch sizes
 // from (n, n_grid) arrays, which must be those the workspace was initialised
@@ -83,7 +83,7 @@ int make_plan(int32_t S, const int64_t *n, const int32_t *ng, BatchPlan &bp) {
     bp.off_sblk = o;  o = pm::align_up(o + arr, A);
     bp.off_gblk = o;  o = pm::align_up(o + arr, A);
     bp.off_ctab = o;  o = pm::align_up(o + arr, A);
-    bp.L = pm::make_layout_sized(bp.n_total, bp.n_nodes, bp.n_gblocks, key_bits, S, o);
+    bp.L = pm::make_layout_sized(bp.n_total, bp.n_nodes, bp.n_gblocks, bp.n_sblocks, key_bits, S, o);
     bp.off_prms += bp.L.tables;
     bp.off_pb += bp.L.tables;
     bp.off_nodeb += bp.L.tables;
@@ -257,11 +257,8 @@ int pm_batch_substep(int32_t n_scenes, const int64_t *n, const int32_t *n_grid, 
     cudaStream_t s = (cudaStream_t)stream;
     pm::launch_set_clock_batch(sc, w, dev_clocks, s);
     if (bp.n_total > 0) {
-        pm::launch_keys(sc, w, parts, s);
-        pm::launch_sort(w, bp.n_total, s, w.inv_perm, true);
         const WsRecord knobs = recorded_knobs(ws);
-        pm::launch_p2g(sc, parts, w, s, knobs.p2g_ctas, knobs.stress_ctas);
-        pm::launch_compact(w, s);
+        pm::launch_p2g(sc, parts, w, s, bp.n_ctas, knobs.p2g_ctas, knobs.stress_ctas);
         pm::launch_grid(sc, w, s, knobs.grid_ctas);
         pm::launch_g2p(sc, parts, w, s, bp.n_ctas, knobs.g2p_ctas);
     }

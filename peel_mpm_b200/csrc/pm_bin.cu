@@ -1,6 +1,6 @@
-// Particle binning: per-substep cell keys and a stable LSD radix sort of
-// (key, particle id), and the compaction of the active 4^3 grid blocks that
-// P2G marks.
+// Particle binning as a whole sort: cell keys and a stable LSD radix sort of
+// (key, particle id), for pm_bin, pm_bin_sort and the renderer's median.  The
+// substep itself bins by counting (k_count, k_offsets in pm_p2g.cu).
 //
 // Key = _node_index(base) of the quadratic base cell (anisompm.py:544-548,
 // 586-590), x-major with z fastest.  The permutation equals the stable
@@ -27,99 +27,6 @@ __global__ void __launch_bounds__(256) k_keys(const float *__restrict__ x, long 
         if (allow != nullptr && allow[p]) any = true;
     }
     if (__any_sync(0xffffffffu, any) && (threadIdx.x & 31) == 0 && ctrl != nullptr) ctrl->any_allow = 1;
-}
-
-// Substep keys: block-major sort key of the base cell, offset by the scene's
-// first sort block; identity ids; allow.any() per scene; and the first radix
-// pass's digit histogram.  One CTA per radix tile (kSortTile particles), so the
-// tile's histogram column is complete when the CTA ends; each thread takes
-// particles t, t + 256, ... of the tile, four at a time with their loads
-// issued together.
-template <class SC>
-__global__ void __launch_bounds__(kSortThreads) k_keys_t(const SC sc, const float *__restrict__ x, long long n,
-                                                         long long ps, unsigned *__restrict__ keys,
-                                                         int *__restrict__ vals, const unsigned char *__restrict__ allow,
-                                                         Ctrl *ctrl, unsigned *__restrict__ hist, int n_tiles) {
-    __shared__ unsigned cnt[kRadix];
-    for (int i = threadIdx.x; i < kRadix; i += kSortThreads) cnt[i] = 0;
-    __syncthreads();
-    const long long t0 = (long long)blockIdx.x * kSortTile;
-    const int lane = threadIdx.x & 31;
-    bool any_plain = false;
-    int sid = 0;
-    if (SC::batched) sid = sc.of_particle(min(t0 + threadIdx.x, n - 1));
-    constexpr int G = 4;
-#pragma unroll 1
-    for (int k0 = 0; k0 < kSortItems; k0 += G) {
-        float xp[G][3];
-        unsigned char al[G];
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            const long long p = t0 + (long long)(k0 + g) * kSortThreads + threadIdx.x;
-            const bool ok = p < n;
-#pragma unroll
-            for (int a = 0; a < 3; ++a) xp[g][a] = ok ? x[a * ps + p] : 0.0f;
-            al[g] = ok ? allow[p] : (unsigned char)0;
-        }
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            const long long p = t0 + (long long)(k0 + g) * kSortThreads + threadIdx.x;
-            const bool ok = p < n;
-            if (SC::batched && ok) {
-                while (p >= sc.p_end(sid, n)) ++sid;   // particles of a thread come in increasing order
-            }
-            const pm_params &prm = sc.params(sid);
-            const int ng = prm.n_grid;
-            const float inv_dx = (float)prm.inv_dx;
-            int qb[3];
-#pragma unroll
-            for (int a = 0; a < 3; ++a) qb[a] = sat_base(floorf(__fsub_rn(__fmul_rn(xp[g][a], inv_dx), 0.5f)), ng);
-            const unsigned key = (sc.sblock_base(sid) << kSortBlockBits) + blocked_key(qb, ng);
-            if (ok) {
-                keys[p] = key;
-                vals[p] = (int)p;
-                atomicAdd(&cnt[key & (kRadix - 1)], 1u);
-            }
-            const bool a = ok && al[g] != 0;
-            if (SC::batched) {
-                // a warp whose lanes share a scene votes once
-                const int s0 = __shfl_sync(0xffffffffu, sid, 0);
-                if (__all_sync(0xffffffffu, sid == s0)) {
-                    if (__any_sync(0xffffffffu, a) && lane == 0) ctrl[s0].any_allow = 1;
-                } else if (a) {
-                    ctrl[sid].any_allow = 1;
-                }
-            } else {
-                any_plain |= a;
-            }
-        }
-    }
-    if (!SC::batched) {
-        if (__syncthreads_or(any_plain) && threadIdx.x == 0) ctrl->any_allow = 1;
-    } else {
-        __syncthreads();
-    }
-    for (int i = threadIdx.x; i < kRadix; i += kSortThreads) hist[(long long)i * n_tiles + blockIdx.x] = cnt[i];
-}
-
-// Compacts the marked blocks into block_list and clears the marks.
-__global__ void __launch_bounds__(256) k_compact_blocks(unsigned char *__restrict__ block_mask, long long nb,
-                                                        int *__restrict__ block_list, Ctrl *ctrl) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    const long long start = (long long)blockIdx.x * blockDim.x;
-    for (long long base = start; base < nb; base += stride) {
-        const long long b = base + threadIdx.x;
-        const bool on = (b < nb) && block_mask[b];
-        const unsigned ball = __ballot_sync(0xffffffffu, on);
-        unsigned slot0 = 0;
-        if ((threadIdx.x & 31) == 0 && ball) slot0 = atomicAdd(&ctrl->n_active, (unsigned)__popc(ball));
-        slot0 = __shfl_sync(0xffffffffu, slot0, 0);
-        if (on) {
-            const unsigned slot = slot0 + __popc(ball & lanemask_lt());
-            if (slot < (unsigned long long)nb) block_list[slot] = (int)b;   // bounded even without a clock reset
-            block_mask[b] = 0;
-        }
-    }
 }
 
 // ------------------------------------------------------------ radix sort
@@ -331,15 +238,14 @@ void prepare_sort() {
 }
 
 template <int RB>
-static void radix_pass(const WS &w, long long n, int tiles, int shift, bool need_hist, const unsigned *kin,
-                       const int *vin, unsigned *kout, int *vout, int *inv, cudaStream_t s) {
-    if (need_hist) k_radix_hist<RB><<<tiles, kSortThreads, 0, s>>>(kin, n, shift, w.hist, tiles);
+static void radix_pass(const WS &w, long long n, int tiles, int shift, const unsigned *kin, const int *vin, unsigned *kout, int *vout, int *inv, cudaStream_t s) {
+    k_radix_hist<RB><<<tiles, kSortThreads, 0, s>>>(kin, n, shift, w.hist, tiles);
     k_radix_rowscan<<<1u << RB, 256, 0, s>>>(w.hist, tiles, w.dtot);
     k_radix_scatter<RB><<<tiles, kSortThreads, radix_scatter_smem<RB>(), s>>>(kin, vin, kout, vout, n, shift, w.hist,
                                                                              tiles, w.dtot, inv);
 }
 
-void launch_sort(const WS &w, long long n, cudaStream_t s, int *inv, bool hist0_ready) {
+void launch_sort(const WS &w, long long n, cudaStream_t s, int *inv) {
     if (n <= 0) return;
     prepare_sort();
     const int tiles = (int)((n + kSortTile - 1) / kSortTile);
@@ -348,13 +254,11 @@ void launch_sort(const WS &w, long long n, cudaStream_t s, int *inv, bool hist0_
     int shift = 0, rem = w.key_bits;
     for (int pass = 0; pass < w.passes; ++pass) {
         const int rb = radix_digit_bits(rem);
-        // launch_keys leaves the first pass's 8-bit histogram
-        const bool need_hist = pass > 0 || !hist0_ready || rb != kRadixBits;
         int *iv = pass == w.passes - 1 ? inv : nullptr;
         if (rb == kRadixBitsTop)
-            radix_pass<kRadixBitsTop>(w, n, tiles, shift, need_hist, kin, vin, kout, vout, iv, s);
+            radix_pass<kRadixBitsTop>(w, n, tiles, shift, kin, vin, kout, vout, iv, s);
         else
-            radix_pass<kRadixBits>(w, n, tiles, shift, need_hist, kin, vin, kout, vout, iv, s);
+            radix_pass<kRadixBits>(w, n, tiles, shift, kin, vin, kout, vout, iv, s);
         shift += rb;
         rem -= rb;
         unsigned *tk = kin; kin = kout; kout = tk;
@@ -362,19 +266,11 @@ void launch_sort(const WS &w, long long n, cudaStream_t s, int *inv, bool hist0_
     }
 }
 
-template <class SC>
-void launch_keys(const SC &sc, const WS &w, const Parts &P, cudaStream_t s) {
+void launch_keys(const pm_params &prm, const WS &w, const Parts &P, cudaStream_t s) {
     if (P.n <= 0) return;
-    const int tiles = (int)((P.n + kSortTile - 1) / kSortTile);
-    k_keys_t<SC><<<tiles, kSortThreads, 0, s>>>(sc, P.x, P.n, P.ps, w.keys_a, w.vals_a, P.allow, w.ctrl, w.hist,
-                                                tiles);
-}
-template void launch_keys<PlainScenes>(const PlainScenes &, const WS &, const Parts &, cudaStream_t);
-template void launch_keys<BatchScenes>(const BatchScenes &, const WS &, const Parts &, cudaStream_t);
-
-void launch_compact(const WS &w, cudaStream_t s) {
-    const int cb = (int)std::min<long long>((w.n_blocks + 255) / 256, 148LL * 8);
-    k_compact_blocks<<<cb > 0 ? cb : 1, 256, 0, s>>>(w.block_mask, w.n_blocks, w.block_list, w.ctrl);
+    const int blocks = (int)std::min<long long>((P.n + 255) / 256, 148LL * 16);
+    k_keys<<<blocks, 256, 0, s>>>(P.x, P.n, P.ps, prm.n_grid, (float)prm.inv_dx, true, w.keys_a, w.vals_a, P.allow,
+                                  w.ctrl);
 }
 
 void launch_keys_only(const float *x, long long n, long long ps, int ng, float inv_dx, bool blocked, const WS &w,

@@ -179,8 +179,8 @@ int pm_bin(const pm_params *prm, const pm_particles *P, void *ws, size_t ws_byte
     if ((rc = get_ws(ws, ws_bytes, P->n, prm->n_grid, &w))) return rc;
     const pm::Parts parts = pm::make_parts(P);
     cudaStream_t s = (cudaStream_t)stream;
-    pm::launch_keys(pm::PlainScenes{*prm}, w, parts, s);
-    pm::launch_sort(w, P->n, s, w.inv_perm, true);
+    pm::launch_keys(*prm, w, parts, s);
+    pm::launch_sort(w, P->n, s, w.inv_perm);
     return cuda_check("pm_bin");
 }
 
@@ -189,8 +189,12 @@ int pm_p2g(const pm_params *prm, const pm_particles *P, void *ws, size_t ws_byte
     if ((rc = check_device()) || (rc = check_params(prm)) || (rc = check_particles(P, true))) return rc;
     pm::WS w;
     if ((rc = get_ws(ws, ws_bytes, P->n, prm->n_grid, &w))) return rc;
-    pm::launch_p2g(pm::PlainScenes{*prm}, pm::make_parts(P), w, (cudaStream_t)stream, prm->p2g_ctas_per_sm, prm->stress_ctas_per_sm);
-    pm::launch_compact(w, (cudaStream_t)stream);
+    // a piece by itself starts clean, whether or not a clock or a grid update ran since the last one: marks left
+    // over would keep blocks off the new list, counters left over would move the payload's runs
+    cudaMemsetAsync(w.block_mask, 0, (size_t)w.n_blocks, (cudaStream_t)stream);
+    cudaMemsetAsync(&w.ctrl->n_work, 0, 4 * sizeof(unsigned), (cudaStream_t)stream);
+    pm::launch_p2g(pm::PlainScenes{*prm}, pm::make_parts(P), w, (cudaStream_t)stream, -1, prm->p2g_ctas_per_sm,
+                   prm->stress_ctas_per_sm);
     return cuda_check("pm_p2g");
 }
 
@@ -226,10 +230,7 @@ static int substep_common(const pm_params *prm, const pm_particles *P, void *ws,
         pm::launch_set_clock_dev(*prm, w, dev_clocks, row, s);
     if (P->n > 0) {
         const pm::PlainScenes sc{*prm};
-        pm::launch_keys(sc, w, parts, s);
-        pm::launch_sort(w, P->n, s, w.inv_perm, true);
-        pm::launch_p2g(sc, parts, w, s, prm->p2g_ctas_per_sm, prm->stress_ctas_per_sm);
-        pm::launch_compact(w, s);
+        pm::launch_p2g(sc, parts, w, s, -1, prm->p2g_ctas_per_sm, prm->stress_ctas_per_sm);
         pm::launch_grid(sc, w, s, prm->grid_ctas_per_sm);
         pm::launch_g2p(sc, parts, w, s, -1, prm->g2p_ctas_per_sm);
     }
@@ -304,10 +305,7 @@ int pm_substep_record(const pm_params *prm, const pm_particles *P, const pm_part
     pm::launch_set_clock(*prm, w, *clk, s);
     if (P->n > 0) {
         const pm::PlainScenes sc{*prm};
-        pm::launch_keys(sc, w, parts, s);
-        pm::launch_sort(w, P->n, s, w.inv_perm, true);
-        pm::launch_p2g(sc, parts, w, s, prm->p2g_ctas_per_sm, prm->stress_ctas_per_sm);
-        pm::launch_compact(w, s);
+        pm::launch_p2g(sc, parts, w, s, -1, prm->p2g_ctas_per_sm, prm->stress_ctas_per_sm);
         pm::launch_grid(sc, w, s, prm->grid_ctas_per_sm);
         pm::launch_g2p(sc, parts, w, s, -1, prm->g2p_ctas_per_sm);
     }

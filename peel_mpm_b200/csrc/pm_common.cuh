@@ -13,6 +13,18 @@ namespace pm {
 constexpr int kBlockEdge = 4;          // grid block = 4^3 nodes (active-block granularity)
 constexpr int kSortBlock = 8;          // sort block = 8^3 cells (P2G work unit)
 constexpr int kSortBlockBits = 9;      // log2(8^3)
+constexpr int kSortCells = 1 << kSortBlockBits;   // cells of a sort block
+// P2G works on units of 4 x 4 x 8 cells (x, y, z), four to a sort block; cells
+// are numbered x, y, z inside a unit (z fastest), so that a unit's x-layer is a
+// contiguous run of 32 cells.
+constexpr int kUnitCells = 128;
+constexpr int kBlockUnits = kSortCells / kUnitCells;
+// Payload places.  A layer whose 32 cells are filled evenly enough is laid out
+// in rows (row k: the k-th particle of every cell, one place per cell), else
+// cell after cell; rows may take up to kPayPlaces places per particle.
+constexpr int kPayPlaces = 2;
+constexpr int kPayBytes = 68;         // of a place: 4 float4 and 1 float
+constexpr int kCellRows = 1 << 31;    // in a cell's first place: its layer is in rows
 constexpr int kSortThreads = 256;
 constexpr int kSortItems = 16;
 constexpr int kSortTile = kSortThreads * kSortItems;   // keys per radix tile
@@ -38,10 +50,11 @@ constexpr int kG2PThreads = 256;     // G2P particles per CTA
 // a particle mass and of a particle damage; they fix the units of the grid's
 // fixed-point accumulators for the substep (see fix_scale).  The constitutive
 // kernel raises them with atomicMax into kBoundSlots slots per quantity (warps
-// spread over the slots, so the atomics do not queue on one address) and a
-// one-block kernel folds the slots into the bounds.  n_work / work_next: the
-// P2G work list of non-empty 4^3-cell sub-blocks and its dynamic cursor
-// (control block 0 of a batch serves all scenes).
+// spread over the slots, so the atomics do not queue on one address; cleared by
+// the clock kernel) and the P2G kernel folds the slots into the bounds.  n_work
+// / work_next: the P2G work list of non-empty units and its dynamic cursor;
+// run_next, run_end: the places taken from the two ends of the payload (control
+// block 0 of a batch serves all scenes).
 constexpr int kBoundSlots = 128;
 struct Ctrl {
     double time;
@@ -51,11 +64,10 @@ struct Ctrl {
     unsigned nonfinite;
     unsigned dense_subblocks;   // sub-blocks beyond the fixed-point headroom (status error)
     unsigned mom_bound, mass_bound, dmg_bound;
-    unsigned n_work, work_next;
-    unsigned pad_;
+    unsigned n_work, work_next, run_next, run_end;   // (cleared together)
     float col_origin[PM_MAX_COLLIDERS][3];
     float col_vel[PM_MAX_COLLIDERS][3];
-    unsigned bound_slots[3][kBoundSlots];   // zero between substeps
+    unsigned bound_slots[3][kBoundSlots];   // cleared by the clock kernel
 };
 
 __host__ __device__ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -78,15 +90,17 @@ __host__ __device__ inline int blocked_key_bits(int ng) {
 
 struct Layout {
     size_t ctrl, keys_a, keys_b, vals_a, vals_b, hist, block_mask, block_list;
-    size_t g_mom, g_dmg, g_vel, g_gd, payload, inv_perm, work, tables, total;
+    size_t g_mom, g_dmg, g_vel, g_gd, payload, inv_perm, work, slot, cells, utot, split, tables, total;
     int passes, key_bits, n_tiles, nbs;
-    long long n_blocks, n_nodes;
+    long long n_blocks, n_nodes, pay_places;
 };
 
-// n particles, n_nodes grid nodes, n_blocks 4^3 grid blocks, sort keys of
-// key_bits bits, n_ctrl control blocks and table_bytes of scene tables.
-__host__ __device__ inline Layout make_layout_sized(long long n, long long n_nodes, long long n_blocks, int key_bits,
-                                                    int n_ctrl, size_t table_bytes) {
+// n particles, n_nodes grid nodes, n_blocks 4^3 grid blocks, n_sblocks 8^3-cell
+// sort blocks, sort keys of key_bits bits, n_ctrl control blocks and table_bytes
+// of scene tables.
+__host__ __device__ inline Layout make_layout_sized(long long n, long long n_nodes, long long n_blocks,
+                                                    long long n_sblocks, int key_bits, int n_ctrl,
+                                                    size_t table_bytes) {
     Layout L;
     const size_t A = 256;
     L.n_tiles = (int)((n + kSortTile - 1) / kSortTile);
@@ -97,6 +111,7 @@ __host__ __device__ inline Layout make_layout_sized(long long n, long long n_nod
     L.n_blocks = n_blocks;
     L.n_nodes = n_nodes;
     size_t nn = (size_t)(n > 0 ? n : 1);
+    L.pay_places = (kPayPlaces * (long long)nn + 31) / 32 * 32;
     size_t o = 0;
     L.ctrl = o;       o = align_up(o + sizeof(Ctrl) * (size_t)(n_ctrl > 0 ? n_ctrl : 1), A);
     L.keys_a = o;     o = align_up(o + 4 * nn, A);
@@ -110,9 +125,13 @@ __host__ __device__ inline Layout make_layout_sized(long long n, long long n_nod
     L.g_dmg = o;      o = align_up(o + 16 * (size_t)L.n_nodes, A);   // 2 x int64 fixed point per node
     L.g_vel = o;      o = align_up(o + 16 * (size_t)L.n_nodes, A);
     L.g_gd = o;       o = align_up(o + 4 * (size_t)L.n_nodes, A);
-    L.payload = o;    o = align_up(o + 80 * nn, A);
+    L.payload = o;    o = align_up(o + 80 * (size_t)L.pay_places, A);     // 5 float4 parts per place
     L.inv_perm = o;   o = align_up(o + 4 * nn, A);
-    L.work = o;       o = align_up(o + 4 * nn, A);                    // starts of the non-empty sub-blocks
+    L.work = o;       o = align_up(o + 4 * nn, A);                    // the non-empty units
+    L.slot = o;       o = align_up(o + 4 * nn, A);                    // a particle's payload place
+    L.cells = o;      o = align_up(o + 8 * (size_t)kSortCells * (size_t)n_sblocks, A);   // per cell: first place, count
+    L.split = o;      o = align_up(o + (size_t)kSortCells * (size_t)n_sblocks, A);       // per cell, 1 byte
+    L.utot = o;       o = align_up(o + 4 * (size_t)kBlockUnits * (size_t)n_sblocks, A);  // per unit: particles
     L.tables = o;     o = align_up(o + table_bytes, A);
     L.total = o;
     return L;
@@ -123,7 +142,8 @@ __host__ __device__ inline Layout make_layout_sized(long long n, long long n_nod
 __host__ __device__ inline Layout make_layout(long long n, int ng) {
     const int nbs = (ng + kBlockEdge - 1) / kBlockEdge;
     const int kb = sort_bits(ng) > blocked_key_bits(ng) ? sort_bits(ng) : blocked_key_bits(ng);
-    Layout L = make_layout_sized(n, (long long)ng * ng * ng, (long long)nbs * nbs * nbs, kb, 1, 0);
+    const long long nb8 = sort_blocks_per_axis(ng);
+    Layout L = make_layout_sized(n, (long long)ng * ng * ng, (long long)nbs * nbs * nbs, nb8 * nb8 * nb8, kb, 1, 0);
     L.nbs = nbs;
     return L;
 }
@@ -146,11 +166,21 @@ struct WS {
     float *tape_aff;    // APIC affine term, 9 planes (recorded for the adjoint; NULL otherwise)
     float *tape_pol;    // polar R, V, S and phi, 22 planes (recorded for the adjoint; NULL otherwise)
     long long tape_aff_stride;
-    float4 *payload;    // P2G payload, 5 float4 per particle in sorted order
+    void *payload;      // P2G payload in blocks of 32 places (see pm_sweep.cuh)
+    int *ids;           // particle at each payload place, in order of arrival
+    long long pay_places;
     const unsigned *sorted_keys;
     const int *perm;
-    int *inv_perm;      // particle -> sorted position, written by the last radix pass
-    int *work;          // sorted index of the first particle of every non-empty 4^3-cell sub-block
+    int *inv_perm;      // particle -> sorted position, written by the last radix pass of pm_bin
+    int *work;          // the non-empty units
+    int *slot;          // per particle: arrival number in its cell, then payload place
+    int2 *cells;        // per cell (unit_key): {first payload place (and kCellRows), particle count}; zero
+                        // between substeps
+    int *utot;          // per unit: cells reached; zero between substeps
+    unsigned char *split;   // per cell of a listed unit: particles of its 4^3-cell sub-block before it in Morton
+                            // order, mod 256
+    int2 *rec_cells;    // the listed units' cells, kept for the adjoint (NULL otherwise)
+    unsigned char *rec_split;
     int passes, key_bits, n_tiles, nbs;
     long long n_blocks;
 };
@@ -176,7 +206,9 @@ inline WS make_ws(void *base, const Layout &L) {
     w.tape_aff = nullptr;
     w.tape_pol = nullptr;
     w.tape_aff_stride = 0;
-    w.payload = (float4 *)(b + L.payload);
+    w.payload = b + L.payload;
+    w.pay_places = L.pay_places;
+    w.ids = (int *)(b + L.payload + kPayBytes * (size_t)L.pay_places);
     w.passes = L.passes;
     w.key_bits = L.key_bits;
     w.n_tiles = L.n_tiles;
@@ -187,6 +219,12 @@ inline WS make_ws(void *base, const Layout &L) {
     w.perm = (L.passes & 1) ? w.vals_b : w.vals_a;
     w.inv_perm = (int *)(b + L.inv_perm);
     w.work = (int *)(b + L.work);
+    w.slot = (int *)(b + L.slot);
+    w.cells = (int2 *)(b + L.cells);
+    w.utot = (int *)(b + L.utot);
+    w.split = (unsigned char *)(b + L.split);
+    w.rec_cells = nullptr;
+    w.rec_split = nullptr;
     return w;
 }
 
@@ -363,8 +401,7 @@ __device__ __forceinline__ unsigned cell_key(const int b[3], int ng) {
 
 // Morton (z-order) number of a cell inside its 8^3 sort block, bits
 // x2 y2 z2 x1 y1 z1 x0 y0 z0: every aligned run of 8^k numbers is a brick of
-// edge 2^k, and the top three bits name the cell's 4^3-cell sub-block (the
-// P2G work unit).
+// edge 2^k, and the top three bits name the cell's 4^3-cell sub-block.
 __host__ __device__ __forceinline__ unsigned morton9(unsigned x, unsigned y, unsigned z) {
     unsigned m = 0;
 #pragma unroll
@@ -372,14 +409,7 @@ __host__ __device__ __forceinline__ unsigned morton9(unsigned x, unsigned y, uns
         m |= (((x >> b) & 1u) << (3 * b + 2)) | (((y >> b) & 1u) << (3 * b + 1)) | (((z >> b) & 1u) << (3 * b));
     return m;
 }
-// Cell of Morton number m (low 6 bits: inside the 4^3 sub-block; 9 bits: inside the 8^3 block).
-__host__ __device__ __forceinline__ void morton_decode(unsigned m, int c[3]) {
-    c[0] = (int)(((m >> 2) & 1u) | ((m >> 4) & 2u) | ((m >> 6) & 4u));
-    c[1] = (int)(((m >> 1) & 1u) | ((m >> 3) & 2u) | ((m >> 5) & 4u));
-    c[2] = (int)((m & 1u) | ((m >> 2) & 2u) | ((m >> 4) & 4u));
-}
-
-// Sort key of the substep: the same base cell, numbered block-major (8^3-cell
+// Sort key of pm_bin: the same base cell, numbered block-major (8^3-cell
 // blocks in x-major order, cells in Morton order inside a block) so that a
 // run of the sorted order is a compact brick.  A bijection of cell_key.
 __device__ __forceinline__ unsigned blocked_key(const int b[3], int ng) {
@@ -387,6 +417,16 @@ __device__ __forceinline__ unsigned blocked_key(const int b[3], int ng) {
     const unsigned nb = (unsigned)sort_blocks_per_axis(ng);
     const unsigned blk = ((unsigned)(x >> 3) * nb + (unsigned)(y >> 3)) * nb + (unsigned)(z >> 3);
     return (blk << kSortBlockBits) | morton9((unsigned)x & 7u, (unsigned)y & 7u, (unsigned)z & 7u);
+}
+
+// The same cell in the substep's own table: sort block, unit (x2, y2), then the
+// cell inside the unit.
+__device__ __forceinline__ unsigned unit_key(const int b[3], int ng) {
+    const int x = clampi(b[0], 0, ng - 1), y = clampi(b[1], 0, ng - 1), z = clampi(b[2], 0, ng - 1);
+    const unsigned nb = (unsigned)sort_blocks_per_axis(ng);
+    const unsigned blk = ((unsigned)(x >> 3) * nb + (unsigned)(y >> 3)) * nb + (unsigned)(z >> 3);
+    return (((blk << 1) | ((unsigned)x >> 2 & 1u)) << 1 | ((unsigned)y >> 2 & 1u)) << 7 |
+           ((unsigned)x & 3u) << 5 | ((unsigned)y & 3u) << 3 | ((unsigned)z & 7u);
 }
 
 // ------------------------------------------------------- fixed-point grid sums
@@ -483,6 +523,7 @@ __device__ __forceinline__ void mmt3_rn(const float *A, const float *B, float *C
 // the scalar operation would), halving the issue slots of paired arithmetic.
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 bc2(float a) { return make_float2(a, a); }
 
 __device__ __forceinline__ float nan_to_num(float a) {
@@ -683,6 +724,16 @@ __device__ __forceinline__ void qw(float f, float w[3]) {
     w[1] = 0.75f - t1 * t1;
     w[2] = 0.5f * (t2 * t2);
 }
+// cw5's weight of node n (0..4) alone.
+__device__ __forceinline__ float cw5_node(int n, float fx) {
+    const bool s1 = fx >= 1.0f;
+    const float f = s1 ? fx - 1.0f : fx;
+    const int k = s1 ? n - 1 : n;                 // index in the particle's own 4-node stencil
+    const float g = (k & 1) ? f : 1.0f - f;
+    const float g2 = g * g, g3 = g2 * g;
+    const float w = (k == 0 || k == 3) ? (1.0f / 6.0f) * g3 : (2.0f / 3.0f - g2) + 0.5f * g3;
+    return (k < 0 || k > 3) ? 0.0f : w;
+}
 // Cubic weights of one axis expanded onto the 5 nodes [qb-1, qb+3] of a
 // quadratic cell: with s = (fx >= 1) the particle's cubic base is qb - 1 + s
 // and its fraction f = fx - s (both exact), so node n takes weight w[n - s]
@@ -702,6 +753,13 @@ __device__ __forceinline__ void cw5(float fx, float e[5]) {
     e[3] = s1 ? w2 : w3;
     e[4] = s1 ? w3 : 0.0f;
 }
+__device__ __forceinline__ float cw5_2_node(int n, float fx) {   // node n (0..4) alone
+    const bool s1 = fx >= 1.0f;
+    const float f = s1 ? fx - 1.0f : fx;
+    const int k = s1 ? n - 1 : n;
+    const float w = k == 0 ? 1.0f - f : (k == 1 ? 3.0f * f - 2.0f : (k == 2 ? 1.0f - 3.0f * f : f));
+    return (k < 0 || k > 3) ? 0.0f : w;
+}
 __device__ __forceinline__ void cw5_2(float fx, float e[5]) {
     const bool s1 = fx >= 1.0f;
     const float f = s1 ? fx - 1.0f : fx;
@@ -713,26 +771,7 @@ __device__ __forceinline__ void cw5_2(float fx, float e[5]) {
     e[4] = s1 ? w3 : 0.0f;
 }
 
-// A node's fixed-point sum over one chunk of work, split over two 32-bit
-// planes: `lo` sums the low kSplitBits bits of every contribution (unsigned,
-// so at most 2^(32 - kSplitBits) = 256 contributions per node and chunk) and
-// `hi` the rest (q >> kSplitBits, signed; a contribution is below 2^kFixBits
-// per particle, so a chunk of 256 particles keeps |hi| under 2^31).  Both
-// adds are fire-and-forget (no returned value, no carry chain) and
-// unconditional (a branch per add costs more than adding a zero); the pair
-// is folded into an int64 tile, exactly, before either plane can overflow:
-// after every chunk in the adjoint scatter, after every fourth chunk in the
-// forward P2G (whose adds per particle are below 0.42 of 2^kFixBits).
-constexpr int kSplitBits = 24;
-__device__ __forceinline__ void plane_add(unsigned *lo, int *hi, float v, float scale) {
-    const long long q = to_fix(v, scale);
-    atomicAdd(lo, (unsigned)q & ((1u << kSplitBits) - 1u));
-    atomicAdd(hi, (int)(q >> kSplitBits));
-}
-__device__ __forceinline__ long long plane_value(unsigned lo, int hi) {
-    return (long long)hi * (1LL << kSplitBits) + (long long)lo;
-}
-// The same for an entry in global memory: one 64-bit atomic.
+// Adds a value to a fixed-point sum in global memory: one 64-bit atomic.
 __device__ __forceinline__ void red_fix(long long *addr, float v, float scale) {
     const long long q = to_fix(v, scale);
     if (q != 0) atomicAdd((unsigned long long *)addr, (unsigned long long)q);

@@ -15,11 +15,18 @@ __device__ __forceinline__ void reset_ctrl(Ctrl *c, bool shared_counters) {
         c->n_active = 0;
         c->n_work = 0;
         c->work_next = 0;
+        c->run_next = 0;
+        c->run_end = 0;
     }
+}
+__device__ __forceinline__ void clear_bound_slots(Ctrl *c, int t) {   // t: 0 .. kBoundSlots - 1
+#pragma unroll
+    for (int v = 0; v < 3; ++v) c->bound_slots[v][t] = 0u;
 }
 
 __global__ void k_set_clock(Ctrl *c, const pm_clock clk, int ncol) {
     const int t = threadIdx.x;
+    clear_bound_slots(c, t);
     if (t == 0) {
         c->time = clk.time;
         c->step = clk.step;
@@ -38,6 +45,7 @@ __global__ void k_set_clock(Ctrl *c, const pm_clock clk, int ncol) {
 __global__ void k_set_clock_dev(Ctrl *c, const pm_clock *dev, int row, int ncol) {
     const pm_clock *clk = dev + row;
     const int t = threadIdx.x;
+    clear_bound_slots(c, t);
     if (t == 0) {
         c->time = clk->time;
         c->step = clk->step;
@@ -59,6 +67,7 @@ __global__ void k_set_clock_b(Ctrl *c, const pm_params *prms, const pm_clock *de
     const int sid = blockIdx.x, t = threadIdx.x;
     const pm_clock *clk = dev + sid;
     Ctrl *cs = c + sid;
+    clear_bound_slots(cs, t);
     if (t == 0) {
         cs->time = clk->time;
         cs->step = clk->step;
@@ -75,21 +84,22 @@ __global__ void k_set_clock_b(Ctrl *c, const pm_params *prms, const pm_clock *de
 }
 
 void launch_set_clock_batch(const BatchScenes &sc, const WS &w, const pm_clock *dev, cudaStream_t s) {
-    k_set_clock_b<<<sc.n, 32, 0, s>>>(w.ctrl, sc.prms, dev);
+    k_set_clock_b<<<sc.n, kBoundSlots, 0, s>>>(w.ctrl, sc.prms, dev);
 }
 
 void launch_set_clock(const pm_params &prm, const WS &w, const pm_clock &clk, cudaStream_t s) {
-    k_set_clock<<<1, 32, 0, s>>>(w.ctrl, clk, prm.n_colliders);
+    k_set_clock<<<1, kBoundSlots, 0, s>>>(w.ctrl, clk, prm.n_colliders);
 }
 void launch_set_clock_dev(const pm_params &prm, const WS &w, const pm_clock *dev, int row, cudaStream_t s) {
-    k_set_clock_dev<<<1, 32, 0, s>>>(w.ctrl, dev, row, prm.n_colliders);
+    k_set_clock_dev<<<1, kBoundSlots, 0, s>>>(w.ctrl, dev, row, prm.n_colliders);
 }
 
 // ------------------------------------------------------------ grid update
 // One thread per z-row of 4 nodes of an active 4^3 block: the row's scene,
 // parameters and node address are resolved once and its 4 nodes' loads are
-// independent.  Reads and clears the P2G accumulators, writes grid velocity
-// and the normalised damage field (anisompm.py:727-746, 777-779).
+// independent.  Reads and clears the P2G accumulators and the block's mark,
+// writes grid velocity and the normalised damage field (anisompm.py:727-746,
+// 777-779).
 template <class SC>
 __global__ void __launch_bounds__(256) k_grid(const SC sc, const WS w) {
     const long long nact = min((long long)w.ctrl->n_active, w.n_blocks);
@@ -103,6 +113,7 @@ __global__ void __launch_bounds__(256) k_grid(const SC sc, const WS w) {
         const int ng = prm.n_grid, nbs = (ng + kBlockEdge - 1) / kBlockEdge;
         const int b = (int)(gb - sc.gblock_base(sid));
         const int l = (int)(it & 15);
+        if (l == 0) w.block_mask[gb] = 0;   // unmarked for the next substep
         const int bx = b / (nbs * nbs), by = (b / nbs) % nbs, bz = b % nbs;
         const int ix = bx * kBlockEdge + (l >> 2), iy = by * kBlockEdge + (l & 3), iz0 = bz * kBlockEdge;
         if (ix >= ng || iy >= ng) continue;

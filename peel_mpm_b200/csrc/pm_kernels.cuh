@@ -7,18 +7,16 @@
 
 namespace pm {
 
-template <class SC> void launch_keys(const SC &sc, const WS &w, const Parts &P, cudaStream_t s);
-// hist0_ready: the first pass's tile histogram was written by launch_keys
-// (the substep path), so the sort starts at that pass's column scan.
-void launch_sort(const WS &w, long long n, cudaStream_t s, int *inv = nullptr, bool hist0_ready = false);
-void launch_compact(const WS &w, cudaStream_t s);
+void launch_keys(const pm_params &prm, const WS &w, const Parts &P, cudaStream_t s);
+void launch_sort(const WS &w, long long n, cudaStream_t s, int *inv = nullptr);
 void prepare_p2g();
 void prepare_sort();
 void prepare_adjoint();
 void launch_keys_only(const float *x, long long n, long long ps, int ng, float inv_dx, bool blocked, const WS &w,
                       cudaStream_t s);
 template <class SC>
-void launch_p2g(const SC &sc, const Parts &P, const WS &w, cudaStream_t s, int ctas_per_sm = 0, int stress_ctas = 0);
+void launch_p2g(const SC &sc, const Parts &P, const WS &w, cudaStream_t s, long long n_ctas = -1, int ctas_per_sm = 0,
+                int stress_ctas = 0);
 template <class SC> void launch_grid(const SC &sc, const WS &w, cudaStream_t s, int ctas_per_sm = 0);
 void launch_grid_sums(const WS &w, long long n_nodes, float *mom, float *dmg, cudaStream_t s);
 template <class SC>
@@ -26,19 +24,18 @@ void launch_g2p(const SC &sc, const Parts &P, const WS &w, cudaStream_t s, long 
 void launch_set_clock(const pm_params &prm, const WS &w, const pm_clock &clk, cudaStream_t s);
 void launch_set_clock_dev(const pm_params &prm, const WS &w, const pm_clock *dev, int row, cudaStream_t s);
 void launch_set_clock_batch(const BatchScenes &sc, const WS &w, const pm_clock *dev, cudaStream_t s);
-int balanced_range(long long n, int slots, int max_range);
 int resident_slots(const void *kernel, int threads, size_t smem);
 void launch_sym_eig(const float *A, long long n, int sweeps, float *ev, float *V, cudaStream_t s);
 
 // Tape of recorded substeps for the adjoint: a header per slot, the
 // adjoint's control block, its int64 fixed-point scatter grid, two float
 // adjoint grids and its sorted-order payload, shared by all slots; then per
-// slot {v, m} grid, gd, cubic weight sums, the active block list, the sort of
-// the substep (sorted keys, each particle's sorted position, the sub-block
-// work list), the particles' APIC affine term and their polar decomposition
-// (R, V, S) and damage drive phi.
+// slot {v, m} grid, gd, cubic weight sums, the active block list, the binning of
+// the substep (each particle's payload place, the unit list and its cells), the
+// particles' APIC affine term and their polar decomposition (R, V, S) and damage
+// drive phi.
 struct TapeLayout {
-    size_t head, actl, acc, adj_q, adj_c, apay, slot0, vel, gd, sw, vpre, blocks, keys, iperm, work, aff, pol,
+    size_t head, actl, acc, adj_q, adj_c, apay, slot0, vel, gd, sw, vpre, blocks, iperm, work, cells, split, aff, pol,
         slot_bytes, total;
     long long n_blocks, aff_stride;
     int slots, flags;

@@ -1,47 +1,36 @@
-// Constitutive update + P2G, cell-aggregated, in two kernels.
+// Binning, constitutive update and P2G.
+//
+// Binning is by counting, in a table over the substep's cells: k_count gives
+// every particle its arrival number in its cell and lists the non-empty units
+// (4 x 4 x 8 cells), k_offsets gives every unit's cells their payload places,
+// k_place and k_rank turn arrival numbers into places in id order, so that what
+// follows does not depend on the order of arrival.  (A stable radix sort of cell
+// keys took 9 or 10 latency-bound launches, 90 us of the 1M-particle substep,
+// against 50 here.)
 //
 // k_stress, one thread per particle in particle order (coalesced state
 // reads): particle BC, polar decomposition (Jacobi eigensolve of F^T F),
 // fixed-corotated Kirchhoff stress, anisotropic phase-field damage (the
 // Cauchy stress's eigensystem taken from the polar decomposition, a Jacobi
 // solve only for nearly singular F), degradation and the APIC affine term;
-// the P2G payload (5 float4) goes to the particle's slot in the sorted order,
-// and the substep's bounds on one node contribution (momentum, mass, damage)
-// are raised in the control block.
+// the P2G payload goes to the particle's place, and the substep's bounds on one
+// node contribution (momentum, mass, damage) are raised in the control block.
 //
-// k_p2g_tiles, persistent CTAs taking work items from a list of the
-// non-empty 4^3-cell sub-blocks of the sort (the cells of a sub-block are a
-// contiguous run of the Morton-ordered sort).  A work item covers the
-// quadratic nodes [4s, 4s+6)^3 ({mv, m}) and the cubic nodes [4s-1, 4s+7)^3
-// ({sum w d, sum w}).  Chunks of 256 particles stage their payload in shared
-// memory, then one work item per (cell, x-slab): all particles of a cell
-// share their quadratic base, so an item sums the cell's contributions to 9
-// quadratic nodes (3 slabs) or 25 cubic nodes (5 slabs; a cell's cubic
-// stencils span 5^3 nodes) in float registers (packed pairs: sm_100's FFMA2
-// issues two FMAs per instruction), in the sorted order, and adds each node
-// once as exact fixed point (units from the control block's bounds) into two
-// 32-bit shared planes per component.  Every fourth chunk and after the last
-// one the planes go to the global int64 grid, one atomic per nonzero node
-// and component; integer addition is associative, so the grid sums, and with
-// them the whole substep, are the same bits whatever order the atomics run
-// in.  The touched 4^3 grid blocks are marked.  Particles whose stencil needs
-// the reference's edge clamping (base cell outside [1, n_grid-4]) scatter
+// k_p2g_sweep, persistent CTAs taking units from the list: every cell's
+// contributions to its 27 quadratic ({mv, m}) and 125 cubic ({sum w d, sum w})
+// nodes are summed in float registers by a sweep along x and added as exact fixed
+// point (pm_sweep.cuh); integer addition is associative, so the grid sums, and
+// with them the whole substep, are the same bits whatever order the atomics run
+// in.  The 4^3 grid blocks touched are marked and listed.  Particles whose stencil
+// needs the reference's edge clamping (base cell outside [1, n_grid-4]) scatter
 // directly to the global grid instead.
 //
 // Reference: anisompm.py:601-724 (constitutive, damage, P2G) and 768-776
 // (cubic damage scatter).
 #include "pm_kernels.cuh"
+#include "pm_sweep.cuh"
 
 namespace pm {
-
-constexpr int kP2GThreads = 256;
-constexpr int kPay = 17;         // payload floats: x(3) mv(3) affine(9) m d
-// Payload rows are padded by one word per 32 particles: the lanes of an item
-// warp read particle j of 32 different cells, whose sorted positions are
-// close to multiples of the cell occupancy (8): unpadded, those fall on 4
-// banks; padded, on distinct ones.
-constexpr int kPayStride = kP2GThreads + kP2GThreads / 32;
-__device__ __forceinline__ int pay_col(int j) { return j + (j >> 5); }
 
 __device__ __forceinline__ float clamp_min(float v, float lo) { return v < lo ? lo : v; }   // torch.clamp(min=)
 __device__ __forceinline__ float relu(float v) { return v > 0.0f ? v : (v != v ? v : 0.0f); }
@@ -246,23 +235,216 @@ __device__ __forceinline__ void constitutive(const pm_params &prm, const Parts &
     }
 }
 
+// ------------------------------------------------------------------ binning
+// Key of particle p's cell in the substep's cell table.
+template <class SC>
+__device__ __forceinline__ unsigned cell_of(const SC &sc, int sid, const float xp[3], int ng, float inv_dx) {
+    int qb[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) qb[a] = sat_base(floorf(__fsub_rn(__fmul_rn(xp[a], inv_dx), 0.5f)), ng);
+    return (sc.sblock_base(sid) << kSortBlockBits) + unit_key(qb, ng);
+}
+
+// Particles per cell, in the substep's own cell table: every particle takes
+// its arrival number in its cell (one atomic per warp and cell), the first
+// particle of a unit puts the unit on the work list, and allow.any() is
+// raised.  CTAs are aligned to scenes: 256 particles each, four per thread so
+// that the chains of load, atomic and list entry of four particles overlap.
+constexpr int kCountThreads = 64, kCountItems = 256 / kCountThreads;
+template <class SC>
+__global__ void __launch_bounds__(kCountThreads) k_count(const SC sc, const float *__restrict__ x, long long n,
+                                                         long long ps, const unsigned char *__restrict__ allow,
+                                                         const WS w) {
+    const int sid = sc.of_cta(blockIdx.x), lane = threadIdx.x & 31;
+    const pm_params &prm = sc.params(sid);
+    const long long p0 = sc.p_begin(sid) + ((long long)blockIdx.x - sc.cta_base(sid)) * 256 + threadIdx.x;
+    const long long end = sc.p_end(sid, n);
+    const int ng = prm.n_grid;
+    const float inv_dx = (float)prm.inv_dx;
+    unsigned key[kCountItems], peers[kCountItems];
+    int base[kCountItems];
+    bool any = false;
+#pragma unroll
+    for (int g = 0; g < kCountItems; ++g) {
+        const long long p = p0 + g * kCountThreads;
+        key[g] = 0xffffffffu;
+        if (p < end) {
+            const float xp[3] = {x[p], x[ps + p], x[2 * ps + p]};
+            any |= allow[p] != 0;
+            key[g] = cell_of(sc, sid, xp, ng, inv_dx);
+        }
+    }
+#pragma unroll
+    for (int g = 0; g < kCountItems; ++g) {
+        peers[g] = __match_any_sync(0xffffffffu, key[g]);
+        base[g] = 0;
+        if (p0 + g * kCountThreads < end && lane == __ffs(peers[g]) - 1)
+            base[g] = atomicAdd(&w.cells[key[g]].y, __popc(peers[g]));
+    }
+#pragma unroll
+    for (int g = 0; g < kCountItems; ++g) {
+        const long long p = p0 + g * kCountThreads;
+        const int leader = __ffs(peers[g]) - 1;
+        if (p < end && lane == leader && base[g] == 0 && atomicAdd(&w.utot[key[g] / kUnitCells], 1) == 0) {
+            const unsigned i = atomicAdd(&w.ctrl->n_work, 1u);
+            if (i < (unsigned long long)n) w.work[i] = (int)(key[g] / kUnitCells);   // bounded even without a clock reset
+        }
+        const int b = __shfl_sync(0xffffffffu, base[g], leader);
+        if (p < end) w.slot[p] = b + __popc(peers[g] & lanemask_lt());
+    }
+    // one store per scene in the main: a store per warp queues on the one word
+    if (__syncthreads_or(any) && threadIdx.x == 0 && *(volatile int *)&w.ctrl[sid].any_allow == 0)
+        w.ctrl[sid].any_allow = 1;
+}
+
+// Gives every listed unit's layers (32 cells) a run of payload places and the
+// cells their first place; runs lie in any order (the grid sums are exact).  A
+// layer goes in rows, from the front of the payload, if those take at most
+// kPayPlaces places per particle, else cell after cell, from the back, so that
+// the two never meet.  Also counts the 4^3-cell sub-blocks beyond the fixed-point
+// headroom.  One warp per unit, one lane per cell of a layer.
+template <class SC>
+__global__ void __launch_bounds__(256) k_offsets(const SC sc, const WS w, long long n) {
+    __shared__ int s_morton[8][kUnitCells];
+    const unsigned n_work = min(w.ctrl->n_work, (unsigned)min(n, (long long)0x7fffffff));
+    const int lane = threadIdx.x & 31;
+    int *morton = s_morton[threadIdx.x >> 5];
+    const int y = lane >> 3, z = lane & 7;
+    const int mz = (z >> 2) * 64 + (y >> 1) * 16 + ((z >> 1) & 1) * 8 + (y & 1) * 2 + (z & 1);   // x bits: 32 and 4
+    for (unsigned i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n_work; i += (gridDim.x * blockDim.x) >> 5) {
+        const int u = w.work[i];
+        int2 *cells = w.cells + (long long)u * kUnitCells + lane;
+        int c[kUnitX], first[kUnitX], rows_size = 0, flat_size = 0;
+#pragma unroll
+        for (int x = 0; x < kUnitX; ++x) c[x] = cells[32 * x].y;
+#pragma unroll
+        for (int x = 0; x < kUnitX; ++x) {
+            int incl = c[x];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            const int total = __shfl_sync(0xffffffffu, incl, 31), rows = __reduce_max_sync(0xffffffffu, c[x]);
+            const bool in_rows = rows <= total * kPayPlaces / 32;
+            first[x] = in_rows ? (rows_size + lane) | kCellRows : flat_size + incl - c[x];
+            rows_size += in_rows ? rows * 32 : 0;
+            flat_size += in_rows ? 0 : total;
+        }
+        int base = 0, end = 0;
+        if (lane == 0) {
+            if (rows_size > 0) base = (int)atomicAdd(&w.ctrl->run_next, (unsigned)rows_size);
+            if (flat_size > 0) end = (int)(w.pay_places - atomicAdd(&w.ctrl->run_end, (unsigned)flat_size)) - flat_size;
+        }
+        base = __shfl_sync(0xffffffffu, base, 0);
+        end = __shfl_sync(0xffffffffu, end, 0);
+#pragma unroll
+        for (int x = 0; x < kUnitX; ++x) {
+            const int f = first[x] + (first[x] < 0 ? base : end);
+            cells[32 * x].x = f;
+            if (w.rec_cells) w.rec_cells[(long long)i * kUnitCells + 32 * x + lane] = make_int2(f, c[x]);
+        }
+        {   // particles before each cell in Morton order of its sub-block (16 lanes, 4 cells each, to a sub-block)
+            __syncwarp();
+#pragma unroll
+            for (int x = 0; x < kUnitX; ++x) morton[mz + (x >> 1) * 32 + (x & 1) * 4] = c[x];
+            __syncwarp();
+            int4 m = ((int4 *)morton)[lane];
+            const int sum = m.x + m.y + m.z + m.w;
+            int incl = sum;
+#pragma unroll
+            for (int o = 1; o < 16; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o, 16);
+                if ((lane & 15) >= o) incl += v;
+            }
+            const int before = incl - sum;
+            __syncwarp();
+            ((int4 *)morton)[lane] = make_int4(before, before + m.x, before + m.x + m.y, before + m.x + m.y + m.z);
+            __syncwarp();
+#pragma unroll
+            for (int x = 0; x < kUnitX; ++x) {
+                const unsigned char b = (unsigned char)(morton[mz + (x >> 1) * 32 + (x & 1) * 4] & 255);
+                w.split[(long long)u * kUnitCells + 32 * x + lane] = b;
+                if (w.rec_split) w.rec_split[(long long)i * kUnitCells + 32 * x + lane] = b;
+            }
+        }
+        const int mine = c[0] + c[1] + c[2] + c[3];
+        const int low = __reduce_add_sync(0xffffffffu, (lane & 7) < 4 ? mine : 0);
+        const int high = __reduce_add_sync(0xffffffffu, (lane & 7) < 4 ? 0 : mine);
+        if (lane == 0 && max(low, high) > kDenseSubblock)
+            atomicAdd(&w.ctrl[sc.of_sblock((unsigned)u / kBlockUnits)].dense_subblocks,
+                      (low > kDenseSubblock ? 1u : 0u) + (high > kDenseSubblock ? 1u : 0u));
+    }
+}
+
+// Particle ids by place, in order of arrival.  Particles of cells of more than
+// kRankRows particles are marked in w.slot (see k_rank); those of more than
+// kRankMost, four times what the fixed-point headroom allows a whole sub-block
+// (dense_subblocks reports them; also where positions that are not numbers
+// gather), stay in order of arrival.
+constexpr int kRankRows = 64, kRankWarps = 4, kRankMost = 4 * kDenseSubblock;
+template <class SC>
+__global__ void __launch_bounds__(256) k_place(const SC sc, const float *__restrict__ x, long long n, long long ps,
+                                               const WS w) {
+    const int sid = sc.of_cta(blockIdx.x);
+    const pm_params &prm = sc.params(sid);
+    const long long p = sc.p_begin(sid) + ((long long)blockIdx.x - sc.cta_base(sid)) * 256 + threadIdx.x;
+    if (p >= sc.p_end(sid, n)) return;
+    const float xp[3] = {x[p], x[ps + p], x[2 * ps + p]};
+    const int slot = w.slot[p];
+    const int2 cell = w.cells[cell_of(sc, sid, xp, prm.n_grid, (float)prm.inv_dx)];
+    const long long at = place_of(cell.x, slot);
+    w.ids[at] = (int)p;
+    if (cell.y > kRankRows) w.slot[p] = cell.y > kRankMost ? (int)at : -1;
+}
+
+// Gives every particle its payload place (w.slot): in its cell's run by rank of
+// its id, so that a cell's float sums run over its particles in id order
+// whatever the order of arrival.  One warp per layer, one lane per cell, whose
+// ids it keeps in its own column of shared memory.  Cells of more than kRankRows
+// particles are left to k_stress, where every particle counts for itself (a
+// single lane would take the square of their number alone).  (Counted in k_stress
+// for every cell, reading the ids from global memory: 956 us there against 715
+// and 154 here, 8.8M particles at 27 per cell.)
+__global__ void __launch_bounds__(32 * kRankWarps) k_rank(const WS w, long long n) {
+    __shared__ int s_ids[kRankWarps][kRankRows][32];
+    const unsigned n_layers = min(w.ctrl->n_work, (unsigned)min(n, (long long)0x1fffffff)) * kUnitX;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int (*ids)[32] = s_ids[wid];
+    for (unsigned i = blockIdx.x * kRankWarps + wid; i < n_layers; i += gridDim.x * kRankWarps) {
+        const int2 cell = w.cells[(long long)w.work[i / kUnitX] * kUnitCells + 32 * (i % kUnitX) + lane];
+        const int cnt = cell.y <= kRankRows ? cell.y : 0;
+        const int *src = w.ids + (cell.x & ~kCellRows);
+        const int step = cell.x < 0 ? 32 : 1;
+#pragma unroll 4
+        for (int k = 0; k < cnt; ++k) ids[k][lane] = src[k * step];
+        for (int k = 0; k < cnt; ++k) {
+            const int id = ids[k][lane];
+            int rank = 0;
+#pragma unroll 4
+            for (int j = 0; j < cnt; ++j) rank += ids[j][lane] < id;
+            w.slot[id] = (cell.x & ~kCellRows) + rank * step;
+        }
+    }
+}
+
 // One thread per particle in particle order: particle BC, constitutive update,
 // damage update, degradation and the APIC affine term (anisompm.py:601-713);
-// the P2G payload goes to w.payload[s] (5 float4, coalesced):
-//   {fx | x, m} {m v, d} {affine 0..3} {affine 4..7} {affine 8, regular, 0, 0}
+// the P2G payload goes to the particle's place in its cell, in id order (its
+// rank among the cell's ids: the float sums of a cell then do not depend on the
+// order of arrival in k_count), 4 parts of 16 bytes and one of 4:
+//   {fx | x, d} {m v, m} {a00, a10, a01, a11} {a02, a12, a20, a21} {a22}, a = affine,
 // with fx = X - floor(X - 0.5) per axis for particles whose stencil needs no
-// clamping (regular, base cell in [1, n_grid-4]) and the position x otherwise.
+// clamping (base cell in [1, n_grid-4]) and the position x otherwise.
 // MINB: resident CTAs per SM the registers are budgeted for (3: 80 registers;
 // 4: 64 registers with a few spills), a tunable.
 template <class SC, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_stress(const SC sc, const Parts P, const WS w) {
-    // particle order: the state reads and writes are coalesced; the payload
-    // goes to the particle's sorted position
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= P.n) return;
-    const int sid = sc.of_particle(p);
+    // particle order: the state reads and writes are coalesced; CTAs are aligned to scenes
+    const int sid = sc.of_cta(blockIdx.x);
+    const long long p = sc.p_begin(sid) + ((long long)blockIdx.x - sc.cta_base(sid)) * 256 + threadIdx.x;
+    if (p >= sc.p_end(sid, P.n)) return;
     const pm_params &prm = sc.params(sid);
-    const long long s = w.inv_perm[p];
     const long long ps = P.ps;
     const int ng = prm.n_grid;
     const float inv_dx = (float)prm.inv_dx;
@@ -294,13 +476,31 @@ __global__ void __launch_bounds__(256, MINB) k_stress(const SC sc, const Parts P
     }
     float Cp[9], v[3], xp[3];
 #pragma unroll
+    for (int k = 0; k < 3; ++k) xp[k] = P.x[k * ps + p];
+#pragma unroll
     for (int k = 0; k < 9; ++k) Cp[k] = P.C[k * ps + p];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        v[k] = P.v[k * ps + p];
-        xp[k] = P.x[k * ps + p];
-    }
+    for (int k = 0; k < 3; ++k) v[k] = P.v[k * ps + p];
     const float vol0 = P.vol0[p], m = P.mass[p];
+    float fx[3];
+    bool reg = true;
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+        const float X = __fmul_rn(xp[ax], inv_dx);
+        const float fb = floorf(__fsub_rn(X, 0.5f));
+        reg = reg && (fb >= 1.0f) && (fb <= (float)(ng - 4));
+        fx[ax] = __fsub_rn(X, fb);                                   // in [0.5, 1.5)
+    }
+    long long s = w.slot[p];
+    if (s < 0) {                                                     // a cell of more than kRankRows particles
+        const int2 cell = w.cells[cell_of(sc, sid, xp, ng, inv_dx)];
+        const int *ids = w.ids + (cell.x & ~kCellRows);
+        const long long step = cell.x < 0 ? 32 : 1;
+        int rank = 0;
+        for (int k = 0; k < cell.y; ++k) rank += ids[k * step] < (int)p;
+        s = place_of(cell.x, rank);
+        w.slot[p] = (int)s;                                          // (a recorded substep keeps it)
+    }
     {                                                                // particle BCs (601-602)
         const int g = P.grip_tag ? P.grip_tag[p] : -1;
         if (g >= 0 && g < prm.n_grips) {
@@ -315,21 +515,14 @@ __global__ void __launch_bounds__(256, MINB) k_stress(const SC sc, const Parts P
     float aff[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) aff[k] = coeff * tau[k] + m * Cp[k];
-    float fx[3];
-    bool reg = true;
-#pragma unroll
-    for (int ax = 0; ax < 3; ++ax) {
-        const float X = __fmul_rn(xp[ax], inv_dx);
-        const float fb = floorf(__fsub_rn(X, 0.5f));
-        reg = reg && (fb >= 1.0f) && (fb <= (float)(ng - 4));
-        fx[ax] = __fsub_rn(X, fb);                                   // in [0.5, 1.5)
+    {
+        float4 *dst = (float4 *)pay_at(w.payload, s);
+        dst[0] = reg ? make_float4(fx[0], fx[1], fx[2], d_new) : make_float4(xp[0], xp[1], xp[2], d_new);
+        dst[32] = make_float4(m * v[0], m * v[1], m * v[2], m);
+        dst[64] = make_float4(aff[0], aff[3], aff[1], aff[4]);
+        dst[96] = make_float4(aff[2], aff[5], aff[6], aff[7]);
+        *pay_az2(w.payload, s) = aff[8];
     }
-    float4 *dst = w.payload + 5 * s;
-    dst[0] = reg ? make_float4(fx[0], fx[1], fx[2], m) : make_float4(xp[0], xp[1], xp[2], m);
-    dst[1] = make_float4(m * v[0], m * v[1], m * v[2], d_new);
-    dst[2] = make_float4(aff[0], aff[1], aff[2], aff[3]);
-    dst[3] = make_float4(aff[4], aff[5], aff[6], aff[7]);
-    dst[4] = make_float4(aff[8], reg ? 1.0f : 0.0f, 0.0f, 0.0f);
     {   // bounds of one node contribution: |w (m v + aff dpos)| with w <= 1 and |dpos| <= 1.5 dx per axis
         const float hx = 1.5f * (float)prm.dx;
         float bm = 0.0f;
@@ -341,20 +534,14 @@ __global__ void __launch_bounds__(256, MINB) k_stress(const SC sc, const Parts P
         // any partition of the warp is correct here: each group raises the
         // bounds to its own maximum, in the slot of its warp
         const unsigned am = __activemask();
-        const int slot = (int)(((blockIdx.x << 3) + (threadIdx.x >> 5)) & (kBoundSlots - 1));
-        if (!SC::batched || __all_sync(am, sid == __shfl_sync(am, sid, __ffs(am) - 1))) {
-            bmom = __reduce_max_sync(am, bmom);
-            bmass = __reduce_max_sync(am, bmass);
-            bdmg = __reduce_max_sync(am, bdmg);
-            if ((threadIdx.x & 31) == (unsigned)(__ffs(am) - 1)) {
-                atomicMax(&cw->bound_slots[0][slot], bmom);
-                atomicMax(&cw->bound_slots[1][slot], bmass);
-                atomicMax(&cw->bound_slots[2][slot], bdmg);
-            }
-        } else {
-            atomicMax(&cw->bound_slots[0][slot], bmom);
-            atomicMax(&cw->bound_slots[1][slot], bmass);
-            atomicMax(&cw->bound_slots[2][slot], bdmg);
+        const int bslot = (int)(((blockIdx.x << 3) + (threadIdx.x >> 5)) & (kBoundSlots - 1));
+        bmom = __reduce_max_sync(am, bmom);
+        bmass = __reduce_max_sync(am, bmass);
+        bdmg = __reduce_max_sync(am, bdmg);
+        if ((threadIdx.x & 31) == (unsigned)(__ffs(am) - 1)) {
+            atomicMax(&cw->bound_slots[0][bslot], bmom);
+            atomicMax(&cw->bound_slots[1][bslot], bmass);
+            atomicMax(&cw->bound_slots[2][bslot], bdmg);
         }
     }
     if (w.tape_aff) {
@@ -363,19 +550,29 @@ __global__ void __launch_bounds__(256, MINB) k_stress(const SC sc, const Parts P
     }
 }
 
+// ------------------------------------------------------------------ scatter
+// Marks grid block gb (numbered over all scenes) and says whether it was unmarked.
+__device__ __forceinline__ bool mark_block(unsigned char *mask, long long gb) {
+    const unsigned bit = 1u << (8 * (int)(gb & 3));
+    return (atomicOr((unsigned *)(mask + (gb & ~3LL)), bit) & bit) == 0;
+}
+__device__ __forceinline__ void list_block(const WS &w, long long gb, unsigned slot) {
+    if (slot < (unsigned long long)w.n_blocks) w.block_list[slot] = (int)gb;   // bounded even without a clock reset
+}
+__device__ __forceinline__ void mark_node_block(const WS &w, long long gb0, int nbs, int x, int y, int z) {
+    const long long gb = gb0 + ((long long)(x >> 2) * nbs + (y >> 2)) * nbs + (z >> 2);
+    if (*(volatile unsigned char *)(w.block_mask + gb) == 0 && mark_block(w.block_mask, gb))
+        list_block(w, gb, atomicAdd(&w.ctrl->n_active, 1u));
+}
+
 // Scatter one particle straight into the global grid with the reference's
 // clamped node indices (anisompm.py:716-724, 771-776): the path for particles
 // whose stencil leaves the grid.  `sc` holds the fixed-point scales of
 // {momentum, mass, w d, w}.
-__device__ __forceinline__ void mark_node_block(unsigned char *mask, int nbs, int x, int y, int z) {
-    unsigned char *m = &mask[((long long)(x >> 2) * nbs + (y >> 2)) * nbs + (z >> 2)];
-    if (*m == 0) *m = 1;
-}
-
 __device__ __noinline__ void scatter_particle_global(const float xp[3], const float mv[3], const float aff[9],
                                                      float m, float d, float inv_dx, float dx, int ng,
                                                      const float sc[4], long long *g_mom, long long *g_dmg,
-                                                     unsigned char *mask, int nbs) {
+                                                     const WS &w, long long gb0, int nbs) {
     {
         Quad q;
         quad_weights(xp, inv_dx, ng, q);
@@ -406,7 +603,7 @@ __device__ __noinline__ void scatter_particle_global(const float xp[3], const fl
                     red_fix(g + 1, wk * (mv[1] + a1), sc[0]);
                     red_fix(g + 2, wk * (mv[2] + a2), sc[0]);
                     red_fix(g + 3, wk * m, sc[1]);
-                    mark_node_block(mask, nbs, NX[ox], NY[oy], NZ[oz]);
+                    mark_node_block(w, gb0, nbs, NX[ox], NY[oy], NZ[oz]);
                 }
             }
     }
@@ -431,390 +628,153 @@ __device__ __noinline__ void scatter_particle_global(const float xp[3], const fl
                     long long *g = g_dmg + 2 * (((long long)NX[ox] * ng + NY[oy]) * ng + NZ[oz]);
                     red_fix(g, wk * d, sc[2]);
                     red_fix(g + 1, wk, sc[3]);
-                    mark_node_block(mask, nbs, NX[ox], NY[oy], NZ[oz]);
+                    mark_node_block(w, gb0, nbs, NX[ox], NY[oy], NZ[oz]);
                 }
             }
     }
 }
 
-constexpr int kSubEdge = 4;                    // sub-block edge in cells (the P2G work unit)
-constexpr int kQE = kSubEdge + 2;              // 6: quadratic tile edge, nodes [4s, 4s+6)
-constexpr int kCE = kSubEdge + 4;              // 8: cubic tile edge, nodes [4s-1, 4s+7)
-constexpr int kQN = kQE * kQE * kQE;           // 216
-constexpr int kCN = kCE * kCE * kCE;           // 512
-constexpr int kSub = kP2GThreads;              // particles per chunk
-constexpr int kCW = 15;                        // expanded cubic weights per particle (5 per axis)
-// Chunk planes (32-bit words, one node per word) are laid out with z stride
-// 1, y stride 8 and x stride 52 (quadratic) / 68 (cubic): the 32 cells of a
-// chunk of a sub-block (x in one half, all y and z) then land on 32 distinct
-// banks for every node offset, so a warp of items over distinct cells adds
-// without bank conflicts.
-constexpr int kQSY = 8, kQSX = 52, kQPl = 312;   // 5*52 + 5*8 + 6 = 306 <= 312
-constexpr int kCSY = 8, kCSX = 68, kCPl = 544;   // 7*68 + 7*8 + 8 = 540 <= 544
-constexpr size_t kP2GSmem = sizeof(unsigned) * 2 * (4 * kQPl + 2 * kCPl) +
-                            sizeof(float) * (kPay + kCW) * kPayStride + sizeof(int) * (kSub + 2) + 2 * kSub;
-
-// Folds control block blockIdx.x's bound slots into its three bounds and
-// clears the slots for the next substep.
-__global__ void __launch_bounds__(kBoundSlots) k_bounds(Ctrl *ctrl) {
-    Ctrl *c = ctrl + blockIdx.x;
-    __shared__ unsigned s_m[3][kBoundSlots / 32];
-    const int t = threadIdx.x;
-#pragma unroll
-    for (int v = 0; v < 3; ++v) {
-        const unsigned m = __reduce_max_sync(0xffffffffu, c->bound_slots[v][t]);
-        c->bound_slots[v][t] = 0u;
-        if ((t & 31) == 0) s_m[v][t >> 5] = m;
+template <class SC>
+__global__ void __launch_bounds__(kSweepThreads, 3) k_p2g_sweep(const __grid_constant__ SC sc,
+                                                                const __grid_constant__ WS w, long long n) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    SweepShared &sh = *(SweepShared *)s_raw;
+    int tid;   // read once: the compiler would read the special register again in every row
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
+    const int lane = tid & 31, wid = __reduce_max_sync(0xffffffffu, tid >> 5);
+    Ctrl *ctrl0 = w.ctrl;
+    const unsigned n_units = min(ctrl0->n_work, (unsigned)min(n, (long long)0x1fffffff));
+    const int parts = sweep_parts(n_units), layers = kUnitX / parts;
+    const unsigned n_work = n_units * parts;   // an item is a unit's layers part * layers .. + layers
+    for (int i = tid; i < kSweepQ * 4 * kQRows * kPlaneCols; i += kSweepThreads) sh.qpl[0][0][i] = 0;
+    for (int i = tid; i < kSweepC * 2 * kCRows * kPlaneCols; i += kSweepThreads) sh.cpl[0][0][i] = 0;
+    if (tid < 36) sh.mark[tid] = 0;
+    if (tid == 0) {
+        sh.scale[3] = fix_scale(__float_as_uint(1.0f)).scale;
+        sh.next = sweep_item(atomicAdd(&ctrl0->work_next, 1u), n_work, parts, w.work);
     }
     __syncthreads();
-    if (t < 3) {
-        unsigned m = 0u;
-#pragma unroll
-        for (int k = 0; k < kBoundSlots / 32; ++k) m = max(m, s_m[t][k]);
-        if (t == 0) c->mom_bound = m;
-        if (t == 1) c->mass_bound = m;
-        if (t == 2) c->dmg_bound = m;
-    }
-}
-
-// Sorted index of the first particle of every non-empty 4^3-cell sub-block
-// (where key >> 6 changes), appended in any order: the accumulation is exact,
-// so the order in which work items run does not change the result.
-__global__ void __launch_bounds__(256) k_subblocks(const unsigned *__restrict__ keys, long long n,
-                                                   int *__restrict__ work, Ctrl *ctrl) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long base = (long long)blockIdx.x * blockDim.x; base < n; base += stride) {
-        const long long i = base + threadIdx.x;
-        const bool st = i < n && (i == 0 || (keys[i] >> 6) != (keys[i - 1] >> 6));
-        const unsigned ball = __ballot_sync(0xffffffffu, st);
-        unsigned slot0 = 0;
-        if ((threadIdx.x & 31) == 0 && ball) slot0 = atomicAdd(&ctrl->n_work, (unsigned)__popc(ball));
-        slot0 = __shfl_sync(0xffffffffu, slot0, 0);
-        const unsigned slot = slot0 + __popc(ball & lanemask_lt());
-        if (st && slot < (unsigned long long)n) work[slot] = (int)i;   // bounded even without a clock reset
-    }
-}
-
-// MINB: resident CTAs per SM the registers are budgeted for (3: 80
-// registers; 4: 64 registers with a few spills), a tunable.
-template <class SC, int MINB>
-__global__ void __launch_bounds__(kP2GThreads, MINB) k_p2g_tiles(const SC sc, const WS w, long long n) {
-    extern __shared__ long long s_raw[];
-    unsigned (*qlo)[kQPl] = (unsigned (*)[kQPl])(s_raw);                 // [4][kQPl] chunk planes
-    int (*qhi)[kQPl] = (int (*)[kQPl])(qlo[4]);                         // [4][kQPl]
-    unsigned (*clo)[kCPl] = (unsigned (*)[kCPl])(qhi[4]);                // [2][kCPl]
-    int (*chi)[kCPl] = (int (*)[kCPl])(clo[2]);                         // [2][kCPl]
-    float (*pay)[kPayStride] = (float (*)[kPayStride])(chi[2]);         // [kPay][kPayStride]
-    float (*cwt)[kPayStride] = (float (*)[kPayStride])(pay[kPay]);     // [kCW][kPayStride]
-    int *runs = (int *)(cwt[kCW]);                                      // [kSub + 2]
-    unsigned char *regular = (unsigned char *)(runs + kSub + 2);        // [kSub]
-    unsigned char *lcell = regular + kSub;                              // [kSub] cell inside the sub-block
-    __shared__ int s_wcnt[kP2GThreads / 32];
-    __shared__ unsigned char s_bmark[27];
-    __shared__ unsigned s_item;
-
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const unsigned *keys = w.sorted_keys;
-    Ctrl *ctrl0 = w.ctrl;
-    const unsigned n_work = min(ctrl0->n_work, (unsigned)min(n, (long long)0x7fffffff));
-
-    // the planes start zero; every fold clears what it visits
-    for (int i = tid; i < 2 * (4 * kQPl + 2 * kCPl); i += kP2GThreads) qlo[0][i] = 0u;
-    if (tid < 27) s_bmark[tid] = 0;
-    for (;;) {
-        __syncthreads();                  // the previous item's tiles, marks and shared state are done
-        if (tid == 0) s_item = atomicAdd(&ctrl0->work_next, 1u);
-        __syncthreads();
-        const unsigned item = s_item;
-        if (item >= n_work) break;
-        const long long a = w.work[item];
-        const unsigned key0 = keys[a];
-        const unsigned sbk = key0 >> 6;                      // sub-block id
-        const unsigned gblk = key0 >> kSortBlockBits;        // sub-blocks never span scenes
-        const int sid = sc.of_sblock(gblk);
+    int2 now = sh.next;
+    int scene = -1;
+    __syncthreads();
+    if (tid == 0) sh.next = sweep_item(atomicAdd(&ctrl0->work_next, 1u), n_work, parts, w.work);
+    __syncthreads();
+    if (now.x >= 0 && tid / 32 - now.y < layers && tid / 32 >= now.y)
+        cp_async8(&sh.raw[tid], w.cells + (long long)now.x * kUnitCells + tid);
+    cp_async_commit();
+    while (now.x >= 0) {
+        const int u = now.x, x0 = now.y, x1 = x0 + layers;
+        const unsigned gblk = (unsigned)u / kBlockUnits;
+        const int sid = sc.of_sblock(gblk);                  // sort blocks never span scenes
         const pm_params &prm = sc.params(sid);
-        const Ctrl *cs = w.ctrl + sid;
-        const int ng = prm.n_grid;
-        const int nb = sort_blocks_per_axis(ng);
-        const int nbs = (ng + kBlockEdge - 1) / kBlockEdge;
-        const float inv_dx = (float)prm.inv_dx, dx = (float)prm.dx;
-        const FixScale fm = fix_scale(cs->mom_bound), fma_ = fix_scale(cs->mass_bound),
-                       fd = fix_scale(cs->dmg_bound), fw = fix_scale(__float_as_uint(1.0f));
-        const float scl[4] = {fm.scale, fma_.scale, fd.scale, fw.scale};
+        const int ng = prm.n_grid, nb = sort_blocks_per_axis(ng), nbs = (ng + kBlockEdge - 1) / kBlockEdge;
+        const unsigned blk = gblk - sc.sblock_base(sid);
+        const int org[3] = {(int)(blk / ((unsigned)nb * nb)) * kSortBlock + ((u >> 1) & 1) * kUnitX,
+                            (int)(blk / nb % nb) * kSortBlock + (u & 1) * kUnitY,
+                            (int)(blk % nb) * kSortBlock};   // first cell of the unit
+        if (sid != scene && wid >= 4 && wid < 7) {   // fold the scene's bound slots (kept for the grid update too)
+            unsigned m = 0;
+#pragma unroll
+            for (int k = 0; k < kBoundSlots / 32; ++k) m = max(m, w.ctrl[sid].bound_slots[wid - 4][k * 32 + lane]);
+            m = __reduce_max_sync(0xffffffffu, m);
+            if (lane == 0) {
+                sh.scale[wid - 4] = fix_scale(m).scale;
+                (wid == 4 ? w.ctrl[sid].mom_bound : wid == 5 ? w.ctrl[sid].mass_bound : w.ctrl[sid].dmg_bound) = m;
+            }
+        }
+        scene = sid;
         long long *g_mom = w.g_mom + 4 * sc.node_base(sid);
         long long *g_dmg = w.g_dmg + 2 * sc.node_base(sid);
-        unsigned char *bmask = w.block_mask + sc.gblock_base(sid);
-        const unsigned blk = gblk - sc.sblock_base(sid);
-        const int bz = (int)(blk % nb), by = (int)((blk / nb) % nb), bx = (int)(blk / ((unsigned)nb * nb));
-        const unsigned oct = (key0 >> 6) & 7u;               // Morton: the sub-block inside its 8^3 block
-        const int org[3] = {bx * kSortBlock + (int)((oct >> 2) & 1u) * kSubEdge,
-                            by * kSortBlock + (int)((oct >> 1) & 1u) * kSubEdge,
-                            bz * kSortBlock + (int)(oct & 1u) * kSubEdge};   // first cell of the sub-block
-
-        long long item_n = 0;                               // particles of the sub-block
-        int chunk = 0;
-        for (long long sub = a;; sub += kSub, ++chunk) {
-            // ---------------- the chunk's payload (written by k_stress in sorted
-            // order) into shared memory: coalesced float4 loads
-            const long long i = sub + tid;
-            const unsigned key = i < n ? keys[i] : 0xffffffffu;
-            const bool valid = i < n && (key >> 6) == sbk;
-            if (valid) {
-                const float4 *src = w.payload + 5 * i;
-                const float4 q0 = src[0], q1 = src[1], q2 = src[2], q3 = src[3], q4 = src[4];
-                const int t = pay_col(tid);
-                pay[0][t] = q0.x; pay[1][t] = q0.y; pay[2][t] = q0.z; pay[15][t] = q0.w;
-                pay[3][t] = q1.x; pay[4][t] = q1.y; pay[5][t] = q1.z; pay[16][t] = q1.w;
-                pay[6][t] = q2.x; pay[7][t] = q2.y; pay[8][t] = q2.z; pay[9][t] = q2.w;
-                pay[10][t] = q3.x; pay[11][t] = q3.y; pay[12][t] = q3.z; pay[13][t] = q3.w;
-                pay[14][t] = q4.x;
-                regular[tid] = q4.y != 0.0f ? 1 : 0;
-                lcell[tid] = (unsigned char)(key & 63u);
-                if (q4.y != 0.0f) {   // the cubic weights of the cell's 5 node layers, once per particle
-                    float e[5];
-                    cw5(q0.x, e);
-#pragma unroll
-                    for (int k = 0; k < 5; ++k) cwt[k][t] = e[k];
-                    cw5(q0.y, e);
-#pragma unroll
-                    for (int k = 0; k < 5; ++k) cwt[5 + k][t] = e[k];
-                    cw5(q0.z, e);
-#pragma unroll
-                    for (int k = 0; k < 5; ++k) cwt[10 + k][t] = e[k];
-                }
-            }
-            // runs of equal cell key inside the chunk (ordered compaction), and
-            // the chunk's particle count (the valid lanes are a prefix)
-            int nruns, cnt;
-            {
-                const unsigned prev = (tid > 0 && i <= n) ? keys[i - 1] : 0xffffffffu;
-                const bool flag = valid && (tid == 0 || key != prev);
-                const unsigned fb = __ballot_sync(0xffffffffu, flag), vb = __ballot_sync(0xffffffffu, valid);
-                if (lane == 0) s_wcnt[wid] = (int)(__popc(fb) | (__popc(vb) << 16));
-                __syncthreads();
-                int pos = __popc(fb & lanemask_lt()), tot = 0, vt = 0;
-#pragma unroll
-                for (int w2 = 0; w2 < kP2GThreads / 32; ++w2) {
-                    const int c = s_wcnt[w2];
-                    pos += (w2 < wid) ? (c & 0xffff) : 0;
-                    tot += c & 0xffff;
-                    vt += c >> 16;
-                }
-                if (flag) runs[pos] = tid;
-                if (tid == 0) runs[tot] = vt;
-                nruns = tot;
-                cnt = vt;
-                item_n += vt;
-                __syncthreads();
-            }
-            // ---------------- particles that need clamped nodes
-            if (valid && !regular[tid]) {
-                const int t = pay_col(tid);
-                const float xp[3] = {pay[0][t], pay[1][t], pay[2][t]};   // positions for these particles
-                const float mv[3] = {pay[3][t], pay[4][t], pay[5][t]};
-                float aff[9];
-#pragma unroll
-                for (int k = 0; k < 9; ++k) aff[k] = pay[6 + k][t];
-                scatter_particle_global(xp, mv, aff, pay[15][t], pay[16][t], inv_dx, dx, ng, scl, g_mom, g_dmg,
-                                        bmask, nbs);
-            }
-            // ---------------- (cell, slab) items into the chunk planes: items
-            // 0 .. 3*nruns-1 are quadratic x-slabs, then 5*nruns cubic x-slabs,
-            // slab-major, so the lanes of a warp mostly run one kind and one
-            // slab over distinct cells (distinct nodes at every step)
-            for (int it = tid; it < nruns * 8; it += kP2GThreads) {
-                const bool quad = it < 3 * nruns;
-                const int k = quad ? it : it - 3 * nruns;
-                const int s8 = k / nruns;
-                const int r = k - s8 * nruns;
-                const int sl = quad ? s8 : 3 + s8;
-                const int ja = runs[r], jb = runs[r + 1];
-                int cq[3];
-                morton_decode(lcell[ja], cq);                    // cell inside the sub-block
-                if (sl == 0) {
-                    // the cell's stencils (quadratic nodes c..c+2, cubic c-1..c+3 per
-                    // axis) span grid blocks s-1+b .. s+b with b = (c > 0): marked
-                    // whatever the sums, so that the grid update writes every node a
-                    // gather reads (a node whose contributions all round to zero
-                    // still gets its zero velocity and damage)
-                    const int b0 = cq[0] > 0, b1 = cq[1] > 0, b2 = cq[2] > 0;
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        s_bmark[((b0 + (k >> 2)) * 3 + b1 + ((k >> 1) & 1)) * 3 + b2 + (k & 1)] = 1;
-                }
-                if (sl < 3) {
-                    const int ox = sl;
-                    // packed pairs: components (0, 1) and (2, mass) of every node
-                    float2 acc[3][3][2];
-#pragma unroll
-                    for (int i2 = 0; i2 < 3; ++i2)
-#pragma unroll
-                        for (int j = 0; j < 3; ++j) acc[i2][j][0] = acc[i2][j][1] = make_float2(0.0f, 0.0f);
-                    const int jend = regular[ja] ? jb : ja;
-                    for (int j = ja; j < jend; ++j) {
-                        const int t = pay_col(j);
-                        const float fx0 = pay[0][t], fx1 = pay[1][t], fx2 = pay[2][t];
-                        float wx[3], wy[3], wz[3];
-                        qw(fx0, wx); qw(fx1, wy); qw(fx2, wz);
-                        const float dxo = ((float)ox - fx0) * dx;
-                        const float m = pay[15][t];
-                        const float2 base01 = fma2(make_float2(pay[6][t], pay[9][t]), bc2(dxo),
-                                                   make_float2(pay[3][t], pay[4][t]));
-                        const float base2 = pay[5][t] + pay[12][t] * dxo;
-                        const float2 ay01 = make_float2(pay[7][t], pay[10][t]), az01 = make_float2(pay[8][t], pay[11][t]);
-                        const float ay2 = pay[13][t], az2 = pay[14][t];
-                        const float wxs = ox == 0 ? wx[0] : (ox == 1 ? wx[1] : wx[2]);
-                        float2 bz[3][2], wz2[3];
-#pragma unroll
-                        for (int oz = 0; oz < 3; ++oz) {
-                            const float dz = ((float)oz - fx2) * dx;
-                            wz2[oz] = bc2(wz[oz]);
-                            bz[oz][0] = mul2(wz2[oz], fma2(az01, bc2(dz), base01));
-                            bz[oz][1] = mul2(wz2[oz], make_float2(base2 + az2 * dz, m));
-                        }
-#pragma unroll
-                        for (int oy = 0; oy < 3; ++oy) {
-                            const float wxy = wxs * wy[oy];
-                            const float wdy = wxy * (((float)oy - fx1) * dx);
-                            const float2 w2 = bc2(wxy);
-                            const float2 ady01 = mul2(bc2(wdy), ay01), ady2 = make_float2(wdy * ay2, 0.0f);
-#pragma unroll
-                            for (int oz = 0; oz < 3; ++oz) {
-                                acc[oy][oz][0] = fma2(ady01, wz2[oz], fma2(w2, bz[oz][0], acc[oy][oz][0]));
-                                acc[oy][oz][1] = fma2(ady2, wz2[oz], fma2(w2, bz[oz][1], acc[oy][oz][1]));
-                            }
-                        }
-                    }
-                    const int nx = cq[0] + ox;
-#pragma unroll
-                    for (int oy = 0; oy < 3; ++oy)
-#pragma unroll
-                        for (int oz = 0; oz < 3; ++oz) {
-                            const int sidx = nx * kQSX + (cq[1] + oy) * kQSY + cq[2] + oz;
-                            plane_add(&qlo[0][sidx], &qhi[0][sidx], acc[oy][oz][0].x, scl[0]);
-                            plane_add(&qlo[1][sidx], &qhi[1][sidx], acc[oy][oz][0].y, scl[0]);
-                            plane_add(&qlo[2][sidx], &qhi[2][sidx], acc[oy][oz][1].x, scl[0]);
-                            plane_add(&qlo[3][sidx], &qhi[3][sidx], acc[oy][oz][1].y, scl[1]);
-                        }
-                } else {
-                    const int nxs = sl - 3;
-                    float2 acw[5][5];   // packed pairs (sum w d, sum w) of every node
-#pragma unroll
-                    for (int i2 = 0; i2 < 5; ++i2)
-#pragma unroll
-                        for (int j = 0; j < 5; ++j) acw[i2][j] = make_float2(0.0f, 0.0f);
-                    const int jend = regular[ja] ? jb : ja;
-                    for (int j = ja; j < jend; ++j) {
-                        const int t = pay_col(j);
-                        const float wxs = cwt[nxs][t];
-                        const float d = pay[16][t];
-                        float2 ez2[5];
-#pragma unroll
-                        for (int k = 0; k < 5; ++k) {
-                            const float ez = cwt[10 + k][t];
-                            ez2[k] = make_float2(d * ez, ez);
-                        }
-#pragma unroll
-                        for (int ny = 0; ny < 5; ++ny) {
-                            const float2 w2 = bc2(wxs * cwt[5 + ny][t]);
-#pragma unroll
-                            for (int nz = 0; nz < 5; ++nz) acw[ny][nz] = fma2(w2, ez2[nz], acw[ny][nz]);
-                        }
-                    }
-                    const int nx = cq[0] + nxs;
-#pragma unroll
-                    for (int ny = 0; ny < 5; ++ny)
-#pragma unroll
-                        for (int nz = 0; nz < 5; ++nz) {
-                            const int sidx = nx * kCSX + (cq[1] + ny) * kCSY + cq[2] + nz;
-                            plane_add(&clo[0][sidx], &chi[0][sidx], acw[ny][nz].x, scl[2]);
-                            plane_add(&clo[1][sidx], &chi[1][sidx], acw[ny][nz].y, scl[3]);
-                        }
-                }
-            }
-            __syncthreads();
-            const bool last = cnt < kSub;                       // uniform: the last chunk of the sub-block
-            // the planes take up to four chunks (1,024 particles) before they
-            // must be folded: one add per node is below 0.42 (the largest
-            // quadratic weight) of 2^46 units per particle, so the high plane
-            // stays under 1024 * 0.42 * 2^22 < 2^31; a node takes at most one
-            // add per covering cell and chunk, fewer than 2^7 adds of 24 bits
-            // into the unsigned low plane
-            if (last || (chunk & 3) == 3) {
-                // ---------------- fold the chunk planes straight into the global
-                // grid, one int64 atomic per nonzero node component, clearing
-                // them.  Integer addition is associative, so a sub-block of more
-                // than four chunks, folded more than once, adds the same total.
-                for (int li = tid; li < kQN; li += kP2GThreads) {
-                    const int tx = li / (kQE * kQE), ty = (li / kQE) % kQE, tz = li % kQE;
-                    const int sidx = tx * kQSX + ty * kQSY + tz;
-                    long long q[4];
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const unsigned lo = qlo[c][sidx];
-                        const int hi = qhi[c][sidx];
-                        q[c] = 0;
-                        if ((lo | (unsigned)hi) != 0u) {
-                            qlo[c][sidx] = 0u;
-                            qhi[c][sidx] = 0;
-                            q[c] = plane_value(lo, hi);
-                        }
-                    }
-                    if ((q[0] | q[1] | q[2] | q[3]) != 0) {
-                        long long *g = g_mom + 4 * (((long long)(org[0] + tx) * ng + (org[1] + ty)) * ng + (org[2] + tz));
-#pragma unroll
-                        for (int c = 0; c < 4; ++c)
-                            if (q[c]) atomicAdd((unsigned long long *)(g + c), (unsigned long long)q[c]);
-                    }
-                }
-                for (int li = tid; li < kCN; li += kP2GThreads) {
-                    const int tx = li >> 6, ty = (li >> 3) & 7, tz = li & 7;
-                    const int sidx = tx * kCSX + ty * kCSY + tz;
-                    long long q[2];
-#pragma unroll
-                    for (int c = 0; c < 2; ++c) {
-                        const unsigned lo = clo[c][sidx];
-                        const int hi = chi[c][sidx];
-                        q[c] = 0;
-                        if ((lo | (unsigned)hi) != 0u) {
-                            clo[c][sidx] = 0u;
-                            chi[c][sidx] = 0;
-                            q[c] = plane_value(lo, hi);
-                        }
-                    }
-                    if ((q[0] | q[1]) != 0) {
-                        long long *g = g_dmg + 2 * (((long long)(org[0] - 1 + tx) * ng + (org[1] - 1 + ty)) * ng +
-                                                    (org[2] - 1 + tz));
-                        if (q[0]) atomicAdd((unsigned long long *)g, (unsigned long long)q[0]);
-                        if (q[1]) atomicAdd((unsigned long long *)(g + 1), (unsigned long long)q[1]);
-                    }
-                }
-            }
-            if (last) break;
-            __syncthreads();                                    // the planes are clear for the next chunk
+        if (tid == kSweepThreads - 1) {
+            sh.ng = ng;
+            sh.dx = (float)prm.dx;
+            sh.g_quad = g_mom + 4 * (((long long)org[0] * ng + org[1]) * ng + org[2]);
+            sh.g_cubic = g_dmg + 2 * (((long long)(org[0] - 1) * ng + org[1] - 1) * ng + org[2] - 1);
         }
-        // a sub-block denser than the fixed-point headroom allows: its nodes'
-        // sums are not guaranteed exact; counted for the status
-        if (tid == 0 && item_n > kDenseSubblock) atomicAdd(&w.ctrl[sid].dense_subblocks, 1u);
-        __syncthreads();
-        if (tid < 27 && s_bmark[tid]) {
-            s_bmark[tid] = 0;
-            const int sbx = org[0] >> 2, sby = org[1] >> 2, sbz = org[2] >> 2;   // the sub-block's grid block
-            const int bxx = sbx - 1 + tid / 9, byy = sby - 1 + (tid / 3) % 3, bzz = sbz - 1 + tid % 3;
-            if (bxx >= 0 && byy >= 0 && bzz >= 0 && bxx < nbs && byy < nbs && bzz < nbs)
-                bmask[((long long)bxx * nbs + byy) * nbs + bzz] = 1;
+        // the unit's cells; the table goes back to zero for the next substep
+        const int2 next = sh.next;
+        bool edge = false;                // particles that need clamped nodes
+        int2 cell = make_int2(0, 0);
+        if (wid >= x0 && wid < x1) {
+            cp_async_wait<0>();
+            cell = sh.raw[tid];
+            w.cells[(long long)u * kUnitCells + tid] = make_int2(0, 0);
+            const int c[3] = {tid >> 5, (tid >> 3) & 3, tid & 7};
+            bool reg = true;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) reg = reg && org[a] + c[a] >= 1 && org[a] + c[a] <= ng - 4;
+            edge = cell.y > 0 && !reg;
+            const int cnt = reg ? cell.y : 0;
+            sh.cell[tid] = make_int2(cell.x, cnt);
+            sh.split[tid] = w.split[(long long)u * kUnitCells + tid];
+            const int rows = __reduce_max_sync(0xffffffffu, cnt);
+            if (lane == 0) sh.layer_rows[wid] = rows;
+            if (cnt > 0) {
+                // the cell's stencils (quadratic nodes c..c+2, cubic c-1..c+3 per
+                // axis) span grid blocks (c-1)/4 .. (c+3)/4: marked whatever the
+                // sums, so that the grid update writes every node a gather reads (a
+                // node whose contributions all round to zero still gets its zero
+                // velocity and damage)
+                const int b0 = c[0] > 0, b1 = c[1] > 0, b2 = (c[2] + 3) >> 2;
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    sh.mark[((b0 + (k >> 2)) * 3 + b1 + ((k >> 1) & 1)) * 4 + b2 + (k & 1)] = 1;
+            }
+        } else if (tid == kUnitCells && x0 == 0) {
+            w.utot[u] = 0;
         }
+        const bool edges = __syncthreads_or(edge);
+        const long long gb0 = sc.gblock_base(sid);
+        // the unit after the next is taken, and the next one's cells are on their way, while this one is swept
+        unsigned take = 0;
+        if (tid == kSweepThreads - 1) take = atomicAdd(&ctrl0->work_next, 1u);
+        if (next.x >= 0 && wid >= next.y && wid < next.y + layers)
+            cp_async8(&sh.raw[tid], w.cells + (long long)next.x * kUnitCells + tid);
+        cp_async_commit();
+        if (edges) {                      // the cell's particles over the lanes of its warp
+            const unsigned eb = __ballot_sync(0xffffffffu, edge);
+            for (unsigned m = eb; m; m &= m - 1) {
+                const int l = __ffs(m) - 1;
+                const int f = __shfl_sync(0xffffffffu, cell.x, l), cnt = __shfl_sync(0xffffffffu, cell.y, l);
+                for (int k = lane; k < cnt; k += 32) {
+                    const long long s = place_of(f, k);
+                    const float4 *p = (const float4 *)pay_at(w.payload, s);
+                    const float4 p0 = p[0], p1 = p[32], p2 = p[64], p3 = p[96];
+                    const float xp[3] = {p0.x, p0.y, p0.z}, mv[3] = {p1.x, p1.y, p1.z};
+                    const float aff[9] = {p2.x, p2.z, p3.x, p2.y, p2.w, p3.y, p3.z, p3.w, *pay_az2(w.payload, s)};
+                    scatter_particle_global(xp, mv, aff, p1.w, p0.w, (float)prm.inv_dx, (float)prm.dx, ng, sh.scale, g_mom,
+                                            g_dmg, w, gb0, nbs);
+                }
+            }
+        }
+        if (wid < kSweepQ)
+            sweep_warp<QuadSums<false>, kSweepQ>(sh, sh.qring[wid], (const char *)w.payload, wid, wid, lane, x0, x1);
+        else
+            sweep_warp<CubicSums, kSweepC>(sh, sh.cring[wid - kSweepQ], (const char *)w.payload, wid, wid - kSweepQ,
+                                             lane, x0, x1);
+        if (tid < 64) {                   // the blocks this unit is the first to touch join the list
+            bool fresh = false;
+            long long gb = 0;
+            if (tid < 36 && sh.mark[tid]) {
+                sh.mark[tid] = 0;
+                const int bx = (org[0] >> 2) - 1 + tid / 12, by = (org[1] >> 2) - 1 + (tid >> 2) % 3,
+                          bz = (org[2] >> 2) - 1 + (tid & 3);
+                if (bx >= 0 && by >= 0 && bz >= 0 && bx < nbs && by < nbs && bz < nbs) {
+                    gb = gb0 + ((long long)bx * nbs + by) * nbs + bz;
+                    fresh = mark_block(w.block_mask, gb);
+                }
+            }
+            const unsigned fb = __ballot_sync(0xffffffffu, fresh);
+            unsigned at = 0;
+            if (lane == 0 && fb) at = atomicAdd(&ctrl0->n_active, (unsigned)__popc(fb));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (fresh) list_block(w, gb, at + __popc(fb & lanemask_lt()));
+        } else if (tid == kSweepThreads - 1) {
+            sh.next = sweep_item(take, n_work, parts, w.work);
+        }
+        __syncthreads();                  // the item's shared state is done with
+        now = next;
     }
-}
-
-// Particles per CTA: equal ranges that fill whole waves of the resident CTA
-// slots, so no SM idles behind a partial last wave.
-int balanced_range(long long n, int slots, int max_range) {
-    if (slots < 1) slots = 1;
-    const long long waves = (n + (long long)slots * max_range - 1) / ((long long)slots * max_range);
-    long long r = (n + slots * waves - 1) / (slots * waves);
-    r = (r + 31) / 32 * 32;
-    return (int)std::max<long long>(32, std::min<long long>(r, max_range));
 }
 
 int resident_slots(const void *kernel, int threads, size_t smem) {
@@ -832,51 +792,49 @@ void prepare_p2g() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(k_p2g_tiles<PlainScenes, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kP2GSmem);
-        cudaFuncSetAttribute(k_p2g_tiles<BatchScenes, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kP2GSmem);
-        cudaFuncSetAttribute(k_p2g_tiles<PlainScenes, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kP2GSmem);
-        cudaFuncSetAttribute(k_p2g_tiles<BatchScenes, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kP2GSmem);
+        cudaFuncSetAttribute(k_p2g_sweep<PlainScenes>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(SweepShared));
+        cudaFuncSetAttribute(k_p2g_sweep<BatchScenes>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(SweepShared));
         done[dev] = 1;
     }
 }
 
-// Persistent P2G CTAs: every resident slot of the device (work items are
-// taken from the list dynamically).  `ctas_per_sm`: 0 = the 80-register
-// kernel with as many CTAs as fit (3 per SM); 4 = the 64-register kernel at 4
-// per SM; 1..3 = the 80-register kernel capped at that many per SM.
+// n_ctas: 256-particle CTAs over all scenes (each scene's particles start a new
+// CTA); the plain form derives it from P.n.  Persistent P2G CTAs: every
+// resident slot of the device (units are taken from the list dynamically), or
+// `ctas_per_sm` (1..3) per SM.
 template <class SC>
-void launch_p2g(const SC &sc, const Parts &P, const WS &w, cudaStream_t s, int ctas_per_sm, int stress_ctas) {
+void launch_p2g(const SC &sc, const Parts &P, const WS &w, cudaStream_t s, long long n_ctas, int ctas_per_sm,
+                int stress_ctas) {
     if (P.n <= 0) return;
     prepare_p2g();
-    const int lb = (int)std::min<long long>((P.n + 255) / 256, 148LL * 8);
-    k_subblocks<<<lb, 256, 0, s>>>(w.sorted_keys, P.n, w.work, w.ctrl);
+    const unsigned ctas = (unsigned)(n_ctas >= 0 ? n_ctas : (P.n + 255) / 256);
+    k_count<SC><<<ctas, kCountThreads, 0, s>>>(sc, P.x, P.n, P.ps, P.allow, w);
+    k_offsets<SC><<<(unsigned)std::min<long long>((P.n + 255) / 256, 148LL * 4), 256, 0, s>>>(sc, w, P.n);
+    k_place<SC><<<ctas, 256, 0, s>>>(sc, P.x, P.n, P.ps, w);
+    k_rank<<<(unsigned)std::min<long long>((P.n + 63) / 64, 148LL * 7), 32 * kRankWarps, 0, s>>>(w, P.n);
     if (stress_ctas == 4)
-        k_stress<SC, 4><<<(unsigned)((P.n + 255) / 256), 256, 0, s>>>(sc, P, w);
+        k_stress<SC, 4><<<ctas, 256, 0, s>>>(sc, P, w);
     else
-        k_stress<SC, 3><<<(unsigned)((P.n + 255) / 256), 256, 0, s>>>(sc, P, w);
-    k_bounds<<<sc.count(), kBoundSlots, 0, s>>>(w.ctrl);
-    static int slots_dev[64][2] = {{0}};
+        k_stress<SC, 3><<<ctas, 256, 0, s>>>(sc, P, w);
+    static int slots_dev[64] = {0};
     int dev = 0;
     cudaGetDevice(&dev);
-    const bool wide = ctas_per_sm >= 4;
-    int slots = (dev >= 0 && dev < 64) ? slots_dev[dev][wide] : 0;
+    int slots = (dev >= 0 && dev < 64) ? slots_dev[dev] : 0;
     if (slots <= 0) {
-        slots = wide ? resident_slots((const void *)k_p2g_tiles<SC, 4>, kP2GThreads, kP2GSmem)
-                     : resident_slots((const void *)k_p2g_tiles<SC, 3>, kP2GThreads, kP2GSmem);
-        if (dev >= 0 && dev < 64) slots_dev[dev][wide] = slots;
+        slots = resident_slots((const void *)k_p2g_sweep<SC>, kSweepThreads, sizeof(SweepShared));
+        if (dev >= 0 && dev < 64) slots_dev[dev] = slots;
     }
-    if (ctas_per_sm > 0 && !wide) {   // the cap
+    if (ctas_per_sm > 0) {   // the cap
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         slots = std::min(slots, sms * ctas_per_sm);
     }
-    const unsigned blocks = (unsigned)std::max<long long>(1, std::min<long long>(slots, (P.n + 63) / 64));
-    if (wide)
-        k_p2g_tiles<SC, 4><<<blocks, kP2GThreads, kP2GSmem, s>>>(sc, w, P.n);
-    else
-        k_p2g_tiles<SC, 3><<<blocks, kP2GThreads, kP2GSmem, s>>>(sc, w, P.n);
+    const unsigned blocks = (unsigned)std::max<long long>(1, std::min<long long>(slots, P.n));
+    k_p2g_sweep<SC><<<blocks, kSweepThreads, sizeof(SweepShared), s>>>(sc, w, P.n);
 }
-template void launch_p2g<PlainScenes>(const PlainScenes &, const Parts &, const WS &, cudaStream_t, int, int);
-template void launch_p2g<BatchScenes>(const BatchScenes &, const Parts &, const WS &, cudaStream_t, int, int);
+template void launch_p2g<PlainScenes>(const PlainScenes &, const Parts &, const WS &, cudaStream_t, long long, int, int);
+template void launch_p2g<BatchScenes>(const BatchScenes &, const Parts &, const WS &, cudaStream_t, long long, int, int);
 
 }  // namespace pm

@@ -334,7 +334,7 @@ RenderLayout make_render_layout(long long n, int width, int height, int r_max) {
     const long long per_axis = 2LL * (r_max > 1 ? r_max : 1) / kTile + 2;
     const long long per = std::min(per_axis, (long long)R.ntx) * std::min(per_axis, (long long)R.nty);
     R.cap = std::max<long long>(1, n * per);
-    R.sort = make_layout_sized(n, 0, 0, 32, 1, 0);
+    R.sort = make_layout_sized(n, 0, 0, 0, 32, 1, 0);
     const size_t A = 256, nn = (size_t)(n > 0 ? n : 1), nt = (size_t)ntiles;
     size_t o = R.sort.total;
     R.sp = o;     o = align_up(o + 48 * nn, A);
