@@ -311,8 +311,7 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_adj_sweep(const __grid_con
     asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
     const int lane = tid & 31, wid = __reduce_max_sync(0xffffffffu, tid >> 5);
     const unsigned n_units = min(head->n_work, (unsigned)min(n, (long long)0x1fffffff));
-    const int parts = sweep_parts(n_units), layers = kUnitX / parts;
-    const unsigned n_work = n_units * parts;   // an item is a unit's layers part * layers .. + layers
+    const SweepItems items = sweep_items(n_units);
     const int ng = prm.n_grid, nb = sort_blocks_per_axis(ng);
     for (int i = tid; i < kSweepQ * 4 * kQRows * kPlaneCols; i += kSweepThreads) sh.qpl[0][0][i] = 0;
     for (int i = tid; i < kSweepC * 2 * kCRows * kPlaneCols; i += kSweepThreads) sh.cpl[0][0][i] = 0;
@@ -327,12 +326,10 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_adj_sweep(const __grid_con
             else actl->lap_bound = m;
         }
     }
-    if (tid == 0) sh.next.x = (int)atomicAdd(&actl->work_next, 1u);
     __syncthreads();
-    unsigned item = (unsigned)sh.next.x;
-    while (item < n_work) {
-        const unsigned i = item / parts;   // place in the list
-        const int u = work[i], x0 = (int)(item - i * parts) * layers, x1 = x0 + layers;
+    int2 now = sweep_item(blockIdx.x, items);   // the first item is the CTA's own
+    while (now.x >= 0) {
+        const int i = now.x, u = work[i], x0 = now.y & 255, x1 = now.y >> 8;
         const unsigned blk = (unsigned)u / kBlockUnits;
         const int org[3] = {(int)(blk / ((unsigned)nb * nb)) * kSortBlock + ((u >> 1) & 1) * kUnitX,
                             (int)(blk / nb % nb) * kSortBlock + (u & 1) * kUnitY, (int)(blk % nb) * kSortBlock};
@@ -359,7 +356,7 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_adj_sweep(const __grid_con
         }
         const bool edges = __syncthreads_or(edge);
         unsigned take = 0;                // the next item is taken while this one is swept
-        if (tid == kSweepThreads - 1) take = atomicAdd(&actl->work_next, 1u);
+        if (tid == kSweepThreads - 1) take = gridDim.x + atomicAdd(&actl->work_next, 1u);
         if (edges) {                      // the cell's particles over the lanes of its warp
             const unsigned eb = __ballot_sync(0xffffffffu, edge);
             for (unsigned m = eb; m; m &= m - 1) {
@@ -380,9 +377,9 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_adj_sweep(const __grid_con
         else
             sweep_warp<CubicLapSums, kSweepC>(sh, sh.cring[wid - kSweepQ], (const char *)pay, wid, wid - kSweepQ, lane, x0,
                                              x1);
-        if (tid == kSweepThreads - 1) sh.next.x = (int)take;
+        if (tid == kSweepThreads - 1) sh.next = sweep_item(take, items);
         __syncthreads();
-        item = (unsigned)sh.next.x;
+        now = sh.next;
     }
 }
 

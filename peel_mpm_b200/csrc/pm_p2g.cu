@@ -400,30 +400,45 @@ __global__ void __launch_bounds__(256) k_place(const SC sc, const float *__restr
 
 // Gives every particle its payload place (w.slot): in its cell's run by rank of
 // its id, so that a cell's float sums run over its particles in id order
-// whatever the order of arrival.  One warp per layer, one lane per cell, whose
-// ids it keeps in its own column of shared memory.  Cells of more than kRankRows
-// particles are left to k_stress, where every particle counts for itself (a
-// single lane would take the square of their number alone).  (Counted in k_stress
-// for every cell, reading the ids from global memory: 956 us there against 715
-// and 154 here, 8.8M particles at 27 per cell.)
+// whatever the order of arrival.  One CTA per layer, one lane per cell, the ids in
+// shared memory, a column per cell; every warp ranks every kRankWarps-th
+// particle of the cells.  (With one warp to a layer the chain of a cell's
+// particles squared was the time where units are few: 34 us for 138k particles
+// at 27 per cell, 11 here; sorting the columns by insertion, or skipping
+// columns that arrived in order, was slower: longer chains.)  Cells of more than
+// kRankRows particles are left to k_stress, where every particle counts for
+// itself.  (Counted in k_stress for every cell, reading the ids from global
+// memory: 956 us there against 715 and 85 here, 8.8M particles at 27 per cell.)
 __global__ void __launch_bounds__(32 * kRankWarps) k_rank(const WS w, long long n) {
-    __shared__ int s_ids[kRankWarps][kRankRows][32];
+    __shared__ int ids[kRankRows][32];
     const unsigned n_layers = min(w.ctrl->n_work, (unsigned)min(n, (long long)0x1fffffff)) * kUnitX;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int (*ids)[32] = s_ids[wid];
-    for (unsigned i = blockIdx.x * kRankWarps + wid; i < n_layers; i += gridDim.x * kRankWarps) {
+    for (unsigned i = blockIdx.x; i < n_layers; i += gridDim.x) {
         const int2 cell = w.cells[(long long)w.work[i / kUnitX] * kUnitCells + 32 * (i % kUnitX) + lane];
         const int cnt = cell.y <= kRankRows ? cell.y : 0;
         const int *src = w.ids + (cell.x & ~kCellRows);
         const int step = cell.x < 0 ? 32 : 1;
+        __syncthreads();                     // the layer before is ranked
 #pragma unroll 4
-        for (int k = 0; k < cnt; ++k) ids[k][lane] = src[k * step];
-        for (int k = 0; k < cnt; ++k) {
-            const int id = ids[k][lane];
-            int rank = 0;
+        for (int k = wid; k < cnt; k += kRankWarps) ids[k][lane] = src[k * step];
+        __syncthreads();
+        for (int k0 = wid; k0 < cnt; k0 += 4 * kRankWarps) {   // four at a time: one read for four comparisons
+            int id[4], rank[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int k = k0 + q * kRankWarps;
+                id[q] = k < cnt ? ids[k][lane] : -1;
+                rank[q] = 0;
+            }
 #pragma unroll 4
-            for (int j = 0; j < cnt; ++j) rank += ids[j][lane] < id;
-            w.slot[id] = (cell.x & ~kCellRows) + rank * step;
+            for (int j = 0; j < cnt; ++j) {
+                const int other = ids[j][lane];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) rank[q] += other < id[q];
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (id[q] >= 0) w.slot[id[q]] = (cell.x & ~kCellRows) + rank[q] * step;
         }
     }
 }
@@ -551,17 +566,17 @@ __global__ void __launch_bounds__(256, MINB) k_stress(const SC sc, const Parts P
 }
 
 // ------------------------------------------------------------------ scatter
-// Marks grid block gb (numbered over all scenes) and says whether it was unmarked.
-__device__ __forceinline__ bool mark_block(unsigned char *mask, long long gb) {
+// Marks grid block gb (numbered over all scenes); 0 if it was unmarked.
+__device__ __forceinline__ unsigned mark_block(unsigned char *mask, long long gb) {
     const unsigned bit = 1u << (8 * (int)(gb & 3));
-    return (atomicOr((unsigned *)(mask + (gb & ~3LL)), bit) & bit) == 0;
+    return atomicOr((unsigned *)(mask + (gb & ~3LL)), bit) & bit;
 }
 __device__ __forceinline__ void list_block(const WS &w, long long gb, unsigned slot) {
     if (slot < (unsigned long long)w.n_blocks) w.block_list[slot] = (int)gb;   // bounded even without a clock reset
 }
 __device__ __forceinline__ void mark_node_block(const WS &w, long long gb0, int nbs, int x, int y, int z) {
     const long long gb = gb0 + ((long long)(x >> 2) * nbs + (y >> 2)) * nbs + (z >> 2);
-    if (*(volatile unsigned char *)(w.block_mask + gb) == 0 && mark_block(w.block_mask, gb))
+    if (*(volatile unsigned char *)(w.block_mask + gb) == 0 && mark_block(w.block_mask, gb) == 0)
         list_block(w, gb, atomicAdd(&w.ctrl->n_active, 1u));
 }
 
@@ -644,26 +659,22 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_p2g_sweep(const __grid_con
     const int lane = tid & 31, wid = __reduce_max_sync(0xffffffffu, tid >> 5);
     Ctrl *ctrl0 = w.ctrl;
     const unsigned n_units = min(ctrl0->n_work, (unsigned)min(n, (long long)0x1fffffff));
-    const int parts = sweep_parts(n_units), layers = kUnitX / parts;
-    const unsigned n_work = n_units * parts;   // an item is a unit's layers part * layers .. + layers
+    const SweepItems items = sweep_items(n_units);
     for (int i = tid; i < kSweepQ * 4 * kQRows * kPlaneCols; i += kSweepThreads) sh.qpl[0][0][i] = 0;
     for (int i = tid; i < kSweepC * 2 * kCRows * kPlaneCols; i += kSweepThreads) sh.cpl[0][0][i] = 0;
     if (tid < 36) sh.mark[tid] = 0;
     if (tid == 0) {
         sh.scale[3] = fix_scale(__float_as_uint(1.0f)).scale;
-        sh.next = sweep_item(atomicAdd(&ctrl0->work_next, 1u), n_work, parts, w.work);
+        sh.next = sweep_unit(gridDim.x + atomicAdd(&ctrl0->work_next, 1u), items, w.work);
     }
-    __syncthreads();
-    int2 now = sh.next;
+    int2 now = sweep_unit(blockIdx.x, items, w.work);    // the first item is the CTA's own
     int scene = -1;
-    __syncthreads();
-    if (tid == 0) sh.next = sweep_item(atomicAdd(&ctrl0->work_next, 1u), n_work, parts, w.work);
-    __syncthreads();
-    if (now.x >= 0 && tid / 32 - now.y < layers && tid / 32 >= now.y)
+    if (now.x >= 0 && wid >= (now.y & 255) && wid < now.y >> 8)
         cp_async8(&sh.raw[tid], w.cells + (long long)now.x * kUnitCells + tid);
     cp_async_commit();
+    __syncthreads();
     while (now.x >= 0) {
-        const int u = now.x, x0 = now.y, x1 = x0 + layers;
+        const int u = now.x, x0 = now.y & 255, x1 = now.y >> 8;
         const unsigned gblk = (unsigned)u / kBlockUnits;
         const int sid = sc.of_sblock(gblk);                  // sort blocks never span scenes
         const pm_params &prm = sc.params(sid);
@@ -725,10 +736,21 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_p2g_sweep(const __grid_con
         }
         const bool edges = __syncthreads_or(edge);
         const long long gb0 = sc.gblock_base(sid);
-        // the unit after the next is taken, and the next one's cells are on their way, while this one is swept
-        unsigned take = 0;
-        if (tid == kSweepThreads - 1) take = atomicAdd(&ctrl0->work_next, 1u);
-        if (next.x >= 0 && wid >= next.y && wid < next.y + layers)
+        // the item after the next is taken, the next one's cells are on their way and the blocks are marked, while
+        // this one is swept
+        unsigned take = 0, was = ~0u;
+        if (tid == kSweepThreads - 1) take = gridDim.x + atomicAdd(&ctrl0->work_next, 1u);
+        int gb = 0;
+        if (tid < 36 && sh.mark[tid]) {
+            sh.mark[tid] = 0;
+            const int bx = (org[0] >> 2) - 1 + tid / 12, by = (org[1] >> 2) - 1 + (tid >> 2) % 3,
+                      bz = (org[2] >> 2) - 1 + (tid & 3);
+            if (bx >= 0 && by >= 0 && bz >= 0 && bx < nbs && by < nbs && bz < nbs) {
+                gb = (int)(gb0 + ((long long)bx * nbs + by) * nbs + bz);
+                was = mark_block(w.block_mask, gb);
+            }
+        }
+        if (next.x >= 0 && wid >= (next.y & 255) && wid < next.y >> 8)
             cp_async8(&sh.raw[tid], w.cells + (long long)next.x * kUnitCells + tid);
         cp_async_commit();
         if (edges) {                      // the cell's particles over the lanes of its warp
@@ -752,25 +774,15 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_p2g_sweep(const __grid_con
         else
             sweep_warp<CubicSums, kSweepC>(sh, sh.cring[wid - kSweepQ], (const char *)w.payload, wid, wid - kSweepQ,
                                              lane, x0, x1);
-        if (tid < 64) {                   // the blocks this unit is the first to touch join the list
-            bool fresh = false;
-            long long gb = 0;
-            if (tid < 36 && sh.mark[tid]) {
-                sh.mark[tid] = 0;
-                const int bx = (org[0] >> 2) - 1 + tid / 12, by = (org[1] >> 2) - 1 + (tid >> 2) % 3,
-                          bz = (org[2] >> 2) - 1 + (tid & 3);
-                if (bx >= 0 && by >= 0 && bz >= 0 && bx < nbs && by < nbs && bz < nbs) {
-                    gb = gb0 + ((long long)bx * nbs + by) * nbs + bz;
-                    fresh = mark_block(w.block_mask, gb);
-                }
-            }
+        if (tid < 64) {                   // the blocks this item is the first to touch join the list
+            const bool fresh = was == 0;
             const unsigned fb = __ballot_sync(0xffffffffu, fresh);
             unsigned at = 0;
             if (lane == 0 && fb) at = atomicAdd(&ctrl0->n_active, (unsigned)__popc(fb));
             at = __shfl_sync(0xffffffffu, at, 0);
             if (fresh) list_block(w, gb, at + __popc(fb & lanemask_lt()));
         } else if (tid == kSweepThreads - 1) {
-            sh.next = sweep_item(take, n_work, parts, w.work);
+            sh.next = sweep_unit(take, items, w.work);
         }
         __syncthreads();                  // the item's shared state is done with
         now = next;
@@ -813,7 +825,7 @@ void launch_p2g(const SC &sc, const Parts &P, const WS &w, cudaStream_t s, long 
     k_count<SC><<<ctas, kCountThreads, 0, s>>>(sc, P.x, P.n, P.ps, P.allow, w);
     k_offsets<SC><<<(unsigned)std::min<long long>((P.n + 255) / 256, 148LL * 4), 256, 0, s>>>(sc, w, P.n);
     k_place<SC><<<ctas, 256, 0, s>>>(sc, P.x, P.n, P.ps, w);
-    k_rank<<<(unsigned)std::min<long long>((P.n + 63) / 64, 148LL * 7), 32 * kRankWarps, 0, s>>>(w, P.n);
+    k_rank<<<(unsigned)std::min<long long>(P.n, 148LL * (2048 / (32 * kRankWarps))), 32 * kRankWarps, 0, s>>>(w, P.n);
     if (stress_ctas == 4)
         k_stress<SC, 4><<<ctas, 256, 0, s>>>(sc, P, w);
     else
