@@ -1,6 +1,6 @@
 // Particle binning as a whole sort: cell keys and a stable LSD radix sort of
-// (key, particle id), for pm_bin, pm_bin_sort and the renderer's median.  The
-// substep itself bins by counting (k_count, k_offsets in pm_p2g.cu).
+// (key, particle id), for pm_bin and pm_bin_sort.  The substep itself bins by
+// counting (k_count, k_offsets in pm_p2g.cu).
 //
 // Key = _node_index(base) of the quadratic base cell (anisompm.py:544-548,
 // 586-590), x-major with z fastest.  The permutation equals the stable
@@ -238,7 +238,8 @@ void prepare_sort() {
 }
 
 template <int RB>
-static void radix_pass(const WS &w, long long n, int tiles, int shift, const unsigned *kin, const int *vin, unsigned *kout, int *vout, int *inv, cudaStream_t s) {
+static void radix_pass(const WS &w, long long n, int tiles, int shift, const unsigned *kin, const int *vin,
+                       unsigned *kout, int *vout, int *inv, cudaStream_t s) {
     k_radix_hist<RB><<<tiles, kSortThreads, 0, s>>>(kin, n, shift, w.hist, tiles);
     k_radix_rowscan<<<1u << RB, 256, 0, s>>>(w.hist, tiles, w.dtot);
     k_radix_scatter<RB><<<tiles, kSortThreads, radix_scatter_smem<RB>(), s>>>(kin, vin, kout, vout, n, shift, w.hist,

@@ -7,12 +7,12 @@
 // Screen tiles of 8x8 pixels.  k_splat_project (one thread per gaussian:
 // camera transform, Jacobian, 2D covariance + 0.3 dilation, conic, radius,
 // culling) packs each drawn splat into 48 bytes and counts it into every tile
-// its (2r+1)^2 footprint square touches; a scan of the tile counts and
-// k_splat_emit build per-tile splat lists; k_splat_tiles runs one warp per
+// its (2r+1)^2 footprint square touches; k_tile_alloc and k_splat_emit build
+// per-tile splat lists; k_splat_tiles runs one warp per
 // tile, two pixels per lane: the soft z-buffer walks the tile's list once from
 // shared memory with the pixels' state in registers and each pixel is
 // composed at the end -- no per-pixel atomics, no clear of pixel buffers.
-// tau from the median depth uses the library's radix sort of the depth keys.
+// tau from the median depth selects it digit by digit from the depth keys.
 #include "pm_kernels.cuh"
 
 namespace pm {
@@ -22,16 +22,20 @@ constexpr int kTile = 8;                  // screen tile edge, pixels
 
 struct RenderWS {
     float4 *sp;        // [3n] per splat: {u, v, c00, c01}, {c11, z, u0, v0 (int bits)}, {r, g, b, rad (int bits)}
-    unsigned *count;   // [0] drawn splats, [1] list overflow (never set when the capacity bound holds)
+    unsigned *count;   // [0] drawn splats, [1] list overflow (never set when the capacity bound holds), [2] list length
     float *tau;        // [0] tau, [1] 1 / max(tau, 1e-6)
+    unsigned *keys;    // [n] depth keys (z bits; all ones: not drawn)
+    unsigned *hist;    // [kMedianPasses][kMedianBins] keys by digit, then {prefix, rank, CTAs done per pass}
     unsigned *tcnt;    // [ntiles] splats per tile
-    unsigned *tfill;   // [ntiles] emit cursors
-    unsigned *tstart;  // [ntiles + 1] exclusive prefix of tcnt
+    unsigned *tfill;   // [ntiles] emit cursors, absolute
+    unsigned *tstart;  // [ntiles] first list entry of the tile
     int *tlist;        // [cap] splat ids grouped by tile
     long long cap;
     int ntx, nty;
-    WS sort;           // key / value buffers of the median sort
 };
+
+// The median's digits: 11, 11 and 10 bits from the top.
+constexpr int kMedianPasses = 3, kMedianBins = 2048, kMedianWords = kMedianPasses * kMedianBins + 2 + kMedianPasses;
 
 __device__ __forceinline__ void splat_tiles(int u0, int v0, int rad, int W, int H, int &tx0, int &ty0, int &nx,
                                             int &ny) {
@@ -43,26 +47,28 @@ __device__ __forceinline__ void splat_tiles(int u0, int v0, int rad, int W, int 
     ny = y1 / kTile - ty0 + 1;
 }
 
-__global__ void __launch_bounds__(256) k_splat_clear(RenderWS r, int ntiles) {
+// Clears the counters; tau is the given one, or 1 until a median replaces it.
+__global__ void __launch_bounds__(256) k_splat_clear(RenderWS r, int ntiles, float tau_given) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < 4) r.count[i] = 0;
-    if (i < ntiles) {
-        r.tcnt[i] = 0;
-        r.tfill[i] = 0;
+    if (i < kMedianWords) r.hist[i] = 0;
+    if (i < ntiles) r.tcnt[i] = 0;
+    if (i == 0) {
+        const float tau = tau_given > 0.0f ? tau_given : 1.0f;
+        r.tau[0] = tau;
+        r.tau[1] = 1.0f / (tau > 1e-6f ? tau : 1e-6f);
     }
 }
 
 // Each lane walks the tiles of its own splat; lanes of a warp that hit the
 // same tile in the same step (neighbouring gaussians) add to it with one atomic.
-__device__ __forceinline__ unsigned tile_reserve(unsigned act, unsigned *ctr, int t, bool on) {
-    const unsigned peers = __match_any_sync(act, on ? t : -1);
-    const int leader = __ffs(peers) - 1;
-    const unsigned lane = threadIdx.x & 31;
-    unsigned base = 0;
-    if (on && (int)lane == leader) base = atomicAdd(&ctr[t], (unsigned)__popc(peers));
-    base = __shfl_sync(act, base, leader);
-    return base + (unsigned)__popc(peers & lanemask_lt());
-}
+struct TileWalk {
+    int tx0, ty0, nx, ny, ntx;
+    __device__ __forceinline__ int tile(int k, bool on) const {
+        const int ky = on ? k / nx : 0;
+        return on ? (ty0 + ky) * ntx + tx0 + (k - ky * nx) : -1;
+    }
+};
 
 __global__ void __launch_bounds__(256) k_splat_project(const pm_camera cam, const pm_render_params rp,
                                                        const float *__restrict__ xyz, const float *__restrict__ cov,
@@ -133,94 +139,156 @@ __global__ void __launch_bounds__(256) k_splat_project(const pm_camera cam, cons
     else
         r.sp[3 * i + 2] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(0));
     // depth key for the median of the drawn splats (z > near > 0: the float bits order like the values)
-    r.sort.keys_a[i] = ok ? __float_as_uint(z) : 0xffffffffu;
-    r.sort.vals_a[i] = (int)i;
+    r.keys[i] = ok ? __float_as_uint(z) : 0xffffffffu;
     const unsigned act = __activemask(), drawn = __ballot_sync(act, ok);
     if ((threadIdx.x & 31) == (unsigned)(__ffs(act) - 1) && drawn) atomicAdd(r.count, (unsigned)__popc(drawn));
     // tile counts of the footprint square
-    int tx0 = 0, ty0 = 0, nx = 0, ny = 0;
-    if (ok) splat_tiles(u0, v0, rd, cam.width, cam.height, tx0, ty0, nx, ny);
-    const int nt = nx * ny;
+    TileWalk t{0, 0, 0, 0, r.ntx};
+    if (ok) splat_tiles(u0, v0, rd, cam.width, cam.height, t.tx0, t.ty0, t.nx, t.ny);
+    const int nt = t.nx * t.ny;
     const int steps = __reduce_max_sync(act, nt);
+    const int lane = threadIdx.x & 31;
     for (int k = 0; k < steps; ++k) {
-        const bool on = k < nt;
-        const int ky = on ? k / nx : 0;
-        const int t = on ? (ty0 + ky) * r.ntx + tx0 + (k - ky * nx) : 0;
-        tile_reserve(act, r.tcnt, t, on);
+        const int tile = t.tile(k, k < nt);
+        const unsigned peers = __match_any_sync(act, tile);
+        if (tile >= 0 && lane == __ffs(peers) - 1) atomicAdd(&r.tcnt[tile], (unsigned)__popc(peers));
     }
 }
 
-// tau = 0.02 * median depth (torch.median: the lower middle element), or the given tau
-__global__ void k_splat_tau(RenderWS r, float tau_given, const unsigned *sorted) {
-    if (threadIdx.x != 0) return;
-    float tau = tau_given;
-    if (!(tau_given > 0.0f)) {
-        const unsigned c = r.count[0];
-        tau = c > 0 ? 0.02f * __uint_as_float(sorted[(c - 1) / 2]) : 1.0f;
-    }
-    r.tau[0] = tau;
-    r.tau[1] = 1.0f / (tau > 1e-6f ? tau : 1e-6f);
-}
-
-// Exclusive scan of the tile counts (one CTA of 1024 threads).
-__global__ void __launch_bounds__(1024) k_tile_scan(RenderWS r, int ntiles) {
-    __shared__ unsigned wsum[32];
-    __shared__ unsigned carry;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    if (tid == 0) carry = 0;
+// tau = 0.02 * median depth of the drawn splats (torch.median: the lower middle
+// element), by selection: one pass over the keys per digit counts those that
+// share the digits found so far, and the last CTA to finish finds the digit that
+// holds the wanted rank.  (A whole radix sort of the keys for this one value took
+// 89 of the 500 us of 262k gaussians; the three passes take 25.)
+constexpr int kMedianThreads = 1024;
+template <int PASS>
+__global__ void __launch_bounds__(kMedianThreads) k_median(RenderWS r, long long n) {
+    constexpr int kShift = PASS == 0 ? 21 : (PASS == 1 ? 10 : 0), kBits = PASS == 2 ? 10 : 11;
+    __shared__ unsigned cnt[kMedianBins], wsum[kMedianThreads / 32];
+    __shared__ bool last;
+    const int tid = threadIdx.x, lane = tid & 31;
+    unsigned *hist = r.hist + PASS * kMedianBins, *sel = r.hist + kMedianPasses * kMedianBins;
+    const unsigned prefix = PASS == 0 ? 0u : sel[0];
+    for (int i = tid; i < kMedianBins; i += kMedianThreads) cnt[i] = 0;
     __syncthreads();
-    for (int base = 0; base < ntiles; base += 1024) {
-        const int i = base + tid;
-        const unsigned v = i < ntiles ? r.tcnt[i] : 0u;
-        unsigned incl = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        if (lane == 31) wsum[wid] = incl;
-        __syncthreads();
-        if (wid == 0) {
-            unsigned w = wsum[lane], wi = w;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned y = __shfl_up_sync(0xffffffffu, wi, o);
-                if (lane >= o) wi += y;
-            }
-            wsum[lane] = wi - w;   // exclusive over warps
-        }
-        __syncthreads();
-        const unsigned c = carry;
-        if (i < ntiles) r.tstart[i] = c + wsum[wid] + incl - v;
-        __syncthreads();
-        if (tid == 1023) carry = c + wsum[wid] + incl;
-        __syncthreads();
+    const long long stride = (long long)gridDim.x * kMedianThreads;
+#pragma unroll 4
+    for (long long base = (long long)blockIdx.x * kMedianThreads; base < n; base += stride) {
+        const unsigned key = base + tid < n ? r.keys[base + tid] : 0u;
+        bool on = base + tid < n;
+        if (PASS > 0) on = on && (key >> (PASS == 1 ? 21 : 10)) == prefix;
+        const int bin = on ? (int)((key >> kShift) & ((1u << kBits) - 1u)) : -1;
+        const unsigned peers = __match_any_sync(0xffffffffu, bin);   // depths share their leading digits
+        if (on && lane == __ffs(peers) - 1) atomicAdd(&cnt[bin], (unsigned)__popc(peers));
     }
-    if (tid == 0) r.tstart[ntiles] = carry;
+    __syncthreads();
+    for (int i = tid; i < kMedianBins; i += kMedianThreads)
+        if (cnt[i]) atomicAdd(&hist[i], cnt[i]);
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) last = atomicAdd(&sel[2 + PASS], 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const unsigned drawn = *(volatile unsigned *)r.count;
+    if (drawn == 0) return;                                // tau stays 1
+    const unsigned rank = PASS == 0 ? (drawn - 1) / 2 : *(volatile unsigned *)(sel + 1);
+    constexpr int kOwn = kMedianBins / kMedianThreads;
+    unsigned c[kOwn], sum = 0;
+#pragma unroll
+    for (int k = 0; k < kOwn; ++k) {
+        c[k] = __ldcg(&hist[kOwn * tid + k]);
+        sum += c[k];
+    }
+    unsigned incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) wsum[tid >> 5] = incl;
+    __syncthreads();
+    unsigned before = incl - sum;
+    for (int k = 0; k < tid >> 5; ++k) before += wsum[k];
+#pragma unroll
+    for (int k = 0; k < kOwn; ++k) {
+        if (rank >= before && rank - before < c[k]) {      // one thread, one bin
+            const unsigned found = (prefix << kBits) | (unsigned)(kOwn * tid + k);
+            sel[0] = found;
+            sel[1] = rank - before;
+            if (PASS == kMedianPasses - 1) {
+                const float tau = 0.02f * __uint_as_float(found);
+                r.tau[0] = tau;
+                r.tau[1] = 1.0f / (tau > 1e-6f ? tau : 1e-6f);
+            }
+        }
+        before += c[k];
+    }
 }
 
-// Per-tile lists: every drawn splat id into each tile of its footprint square.
+// Gives every tile its part of the list: a scan within a CTA's tiles, one atomic
+// per CTA for where they begin (the parts lie in any order).  (One CTA scanning
+// all 14,400 tiles took 16 us, this 3.)
+__global__ void __launch_bounds__(256) k_tile_alloc(RenderWS r, int ntiles) {
+    __shared__ unsigned wsum[8], first;
+    const int tid = threadIdx.x, lane = tid & 31, i = blockIdx.x * 256 + tid;
+    const unsigned v = i < ntiles ? r.tcnt[i] : 0u;
+    unsigned incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) wsum[tid >> 5] = incl;
+    __syncthreads();
+    unsigned before = 0, all = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        before += k < (tid >> 5) ? wsum[k] : 0u;
+        all += wsum[k];
+    }
+    if (tid == 0) first = atomicAdd(r.count + 2, all);
+    __syncthreads();
+    if (i < ntiles) r.tstart[i] = r.tfill[i] = first + before + incl - v;
+}
+
+// Per-tile lists: every drawn splat id into each tile of its footprint square,
+// four tiles at a time, their reservations under way together.  Lanes of a warp
+// that hit the same tile in the same step (neighbouring gaussians) reserve
+// with one atomic.
 __global__ void __launch_bounds__(256) k_splat_emit(const pm_camera cam, long long n, RenderWS r) {
+    constexpr int G = 4;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 p1 = r.sp[3 * i + 1], p2 = r.sp[3 * i + 2];
     const int rd = __float_as_int(p2.w);
-    int tx0 = 0, ty0 = 0, nx = 0, ny = 0;
-    if (rd > 0) splat_tiles(__float_as_int(p1.z), __float_as_int(p1.w), rd, cam.width, cam.height, tx0, ty0, nx, ny);
-    const int nt = nx * ny;
+    TileWalk t{0, 0, 0, 0, r.ntx};
+    if (rd > 0)
+        splat_tiles(__float_as_int(p1.z), __float_as_int(p1.w), rd, cam.width, cam.height, t.tx0, t.ty0, t.nx, t.ny);
+    const int nt = t.nx * t.ny;
     const unsigned act = __activemask();
-    const int steps = __reduce_max_sync(act, nt);
-    for (int k = 0; k < steps; ++k) {
-        const bool on = k < nt;
-        const int ky = on ? k / nx : 0;
-        const int t = on ? (ty0 + ky) * r.ntx + tx0 + (k - ky * nx) : 0;
-        const unsigned slot = tile_reserve(act, r.tfill, t, on);
-        if (on) {
-            const long long at = (long long)r.tstart[t] + slot;
-            if (slot < r.tcnt[t] && at < r.cap)
-                r.tlist[at] = (int)i;
-            else
-                r.count[1] = 1;
+    const int steps = __reduce_max_sync(act, nt), lane = threadIdx.x & 31;
+    for (int k0 = 0; k0 < steps; k0 += G) {
+        int tile[G];
+        unsigned peers[G], base[G];
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            tile[q] = t.tile(k0 + q, k0 + q < nt);
+            peers[q] = __match_any_sync(act, tile[q]);
+            base[q] = 0;
+            if (tile[q] >= 0 && lane == __ffs(peers[q]) - 1)
+                base[q] = atomicAdd(&r.tfill[tile[q]], (unsigned)__popc(peers[q]));
+        }
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            const long long at =
+                (long long)__shfl_sync(act, base[q], __ffs(peers[q]) - 1) + __popc(peers[q] & lanemask_lt());
+            if (tile[q] >= 0) {
+                if (at < r.cap)
+                    r.tlist[at] = (int)i;
+                else
+                    r.count[1] = 1;
+            }
         }
     }
 }
@@ -318,8 +386,7 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_splat_tiles(const pm_camera
 }
 
 struct RenderLayout {
-    Layout sort;
-    size_t sp, count, tau, tcnt, tfill, tstart, tlist, total;
+    size_t sp, count, tau, keys, hist, tcnt, tfill, tstart, tlist, total;
     long long cap;
     int ntx, nty;
 };
@@ -334,15 +401,16 @@ RenderLayout make_render_layout(long long n, int width, int height, int r_max) {
     const long long per_axis = 2LL * (r_max > 1 ? r_max : 1) / kTile + 2;
     const long long per = std::min(per_axis, (long long)R.ntx) * std::min(per_axis, (long long)R.nty);
     R.cap = std::max<long long>(1, n * per);
-    R.sort = make_layout_sized(n, 0, 0, 0, 32, 1, 0);
     const size_t A = 256, nn = (size_t)(n > 0 ? n : 1), nt = (size_t)ntiles;
-    size_t o = R.sort.total;
+    size_t o = 0;
     R.sp = o;     o = align_up(o + 48 * nn, A);
     R.count = o;  o = align_up(o + 16, A);
     R.tau = o;    o = align_up(o + 16, A);
+    R.keys = o;   o = align_up(o + 4 * nn, A);
+    R.hist = o;   o = align_up(o + 4 * kMedianWords, A);
     R.tcnt = o;   o = align_up(o + 4 * nt, A);
     R.tfill = o;  o = align_up(o + 4 * nt, A);
-    R.tstart = o; o = align_up(o + 4 * (nt + 1), A);
+    R.tstart = o; o = align_up(o + 4 * nt, A);
     R.tlist = o;  o = align_up(o + 4 * (size_t)R.cap, A);
     R.total = o;
     return R;
@@ -415,6 +483,8 @@ void launch_render(const pm_camera &cam, const pm_render_params &rp, const float
     r.sp = (float4 *)(b + L.sp);
     r.count = (unsigned *)(b + L.count);
     r.tau = (float *)(b + L.tau);
+    r.keys = (unsigned *)(b + L.keys);
+    r.hist = (unsigned *)(b + L.hist);
     r.tcnt = (unsigned *)(b + L.tcnt);
     r.tfill = (unsigned *)(b + L.tfill);
     r.tstart = (unsigned *)(b + L.tstart);
@@ -422,14 +492,16 @@ void launch_render(const pm_camera &cam, const pm_render_params &rp, const float
     r.cap = L.cap;
     r.ntx = L.ntx;
     r.nty = L.nty;
-    r.sort = make_ws(ws, L.sort);
     const int ntiles = L.ntx * L.nty;
-    k_splat_clear<<<(unsigned)((std::max(ntiles, 4) + 255) / 256), 256, 0, s>>>(r, ntiles);
+    k_splat_clear<<<(unsigned)((std::max(ntiles, kMedianWords) + 255) / 256), 256, 0, s>>>(r, ntiles, rp.tau);
     if (n > 0) k_splat_project<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(cam, rp, xyz, cov, color, n, r);
-    const bool median = !(rp.tau > 0.0f);
-    if (median && n > 0) launch_sort(r.sort, n, s);
-    k_splat_tau<<<1, 32, 0, s>>>(r, rp.tau, r.sort.sorted_keys);
-    k_tile_scan<<<1, 1024, 0, s>>>(r, ntiles);
+    if (!(rp.tau > 0.0f) && n > 0) {
+        const unsigned ctas = (unsigned)std::min<long long>((n + 4 * kMedianThreads - 1) / (4 * kMedianThreads), 148LL);
+        k_median<0><<<ctas, kMedianThreads, 0, s>>>(r, n);
+        k_median<1><<<ctas, kMedianThreads, 0, s>>>(r, n);
+        k_median<2><<<ctas, kMedianThreads, 0, s>>>(r, n);
+    }
+    k_tile_alloc<<<(unsigned)((ntiles + 255) / 256), 256, 0, s>>>(r, ntiles);
     if (n > 0) k_splat_emit<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(cam, n, r);
     k_splat_tiles<<<(unsigned)((ntiles + kTileWarps - 1) / kTileWarps), 32 * kTileWarps, 0, s>>>(cam, rp, r, img,
                                                                                                    ntiles);
