@@ -229,6 +229,13 @@ void launch_grid_sums(const WS &w, long long n_nodes, float *mom, float *dmg, cu
 // (anisompm.py:749-760, 781-803).  A footprint larger than the staging
 // buffers (incoherent particle order), or a particle whose stencil needs the
 // reference's edge clamping, gathers from global memory instead.
+//
+// Bound by latency and instruction issue together (64% of issue slots, 3 of 8 waiting
+// warps on loads).  1M particles: 75 us with scalar sums and one index per node,
+// 71 with packed pairs (the same roundings lane by lane) and constant offsets along
+// z.  Staging the damage field in doubled form, to save a move per node, made it
+// slower where the footprint is large: 8.8M particles at 27 per cell 5,300 us for
+// two substeps against 5,195 before and 5,117 now.
 constexpr int kGTQ = 1200;   // staged quadratic nodes (float4)
 constexpr int kGTC = 2400;   // staged cubic nodes (float)
 
@@ -253,9 +260,8 @@ __device__ __forceinline__ void g2p_particle(const pm_params &prm, const Parts &
 #pragma unroll
         for (int o = 0; o < 4; ++o) {
             if (TILE) {
-                NX[o] = (c.b[0] + o - lo[0] + 1) * cd[1] * cd[2];
+                NX[o] = (c.b[0] + o - lo[0] + 1) * cd[1] * cd[2] + c.b[2] - lo[2] + 1;   // z goes by constants
                 NY[o] = (c.b[1] + o - lo[1] + 1) * cd[2];
-                NZ[o] = c.b[2] + o - lo[2] + 1;
             } else {
                 NX[o] = clampi(c.b[0] + o, 0, ng - 1) * ng * ng;
                 NY[o] = clampi(c.b[1] + o, 0, ng - 1) * ng;
@@ -264,22 +270,21 @@ __device__ __forceinline__ void g2p_particle(const pm_params &prm, const Parts &
         }
 #pragma unroll
         for (int ox = 0; ox < 4; ++ox) {
-            float SA = 0.0f, SA2 = 0.0f, SB = 0.0f;
+            float2 S = make_float2(0.0f, 0.0f);                        // (SA, SB)
+            float SA2 = 0.0f;
 #pragma unroll
             for (int oy = 0; oy < 4; ++oy) {
-                float A = 0.0f, B = 0.0f;
+                float2 AB = make_float2(0.0f, 0.0f);
 #pragma unroll
                 for (int oz = 0; oz < 4; ++oz) {
-                    const int node = NX[ox] + NY[oy] + NZ[oz];
-                    const float gd = TILE ? sc[node] : __ldg(&ggd[node]);
-                    A += c.w[oz][2] * gd;
-                    B += c.w2[oz][2] * gd;
+                    const int node = TILE ? NX[ox] + NY[oy] + oz : NX[ox] + NY[oy] + NZ[oz];
+                    const float2 gd = bc2(TILE ? sc[node] : __ldg(&ggd[node]));
+                    AB = fma2(make_float2(c.w[oz][2], c.w2[oz][2]), gd, AB);
                 }
-                SA += c.w[oy][1] * A;
-                SA2 += c.w2[oy][1] * A;
-                SB += c.w[oy][1] * B;
+                S = fma2(bc2(c.w[oy][1]), AB, S);
+                SA2 += c.w2[oy][1] * AB.x;
             }
-            lap += c.w2[ox][0] * SA + c.w[ox][0] * (SA2 + SB);
+            lap += c.w2[ox][0] * S.x + c.w[ox][0] * (SA2 + S.y);
         }
         lap *= (float)(prm.inv_dx * prm.inv_dx);
     }
@@ -289,9 +294,9 @@ __device__ __forceinline__ void g2p_particle(const pm_params &prm, const Parts &
     //   T[x] = sum_y wy Z0,  Ty[x] = sum_y (wy DY) Z0,  Tz[x] = sum_y wy Zd
     //   v = sum_x wx T,  C_.x = sum_x (wx DX) T,  C_.y = sum_x wx Ty,  C_.z = sum_x wx Tz
     // so every node costs 6 FMAs and one float4 load, every column 9 more.
-    float nv[3] = {0.0f, 0.0f, 0.0f}, nC[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) nC[k] = 0.0f;
+    // Components x and y go as packed pairs, z with its moment (g.w holds g.z
+    // again): (Z0, Zd).z, (T, Tz).z, (v.z, C_zz).
+    float nv[3], nC[9];
     {
         Quad q;
         quad_weights(xp, inv_dx, ng, q);
@@ -300,9 +305,8 @@ __device__ __forceinline__ void g2p_particle(const pm_params &prm, const Parts &
 #pragma unroll
         for (int o = 0; o < 3; ++o) {
             if (TILE) {
-                NX[o] = (q.b[0] + o - lo[0]) * qd[1] * qd[2];
+                NX[o] = (q.b[0] + o - lo[0]) * qd[1] * qd[2] + q.b[2] - lo[2];
                 NY[o] = (q.b[1] + o - lo[1]) * qd[2];
-                NZ[o] = q.b[2] + o - lo[2];
             } else {
                 NX[o] = clampi(q.b[0] + o, 0, ng - 1) * ng * ng;
                 NY[o] = clampi(q.b[1] + o, 0, ng - 1) * ng;
@@ -312,37 +316,46 @@ __device__ __forceinline__ void g2p_particle(const pm_params &prm, const Parts &
             wyd[o] = q.w[o][1] * (((float)o - q.fx[1]) * dx);
             wzd[o] = q.w[o][2] * (((float)o - q.fx[2]) * dx);
         }
+        const float2 zero = make_float2(0.0f, 0.0f);
+        float2 v01 = zero, Cx01 = zero, Cy01 = zero, Cz01 = zero, v2Cz2 = zero;
+        float Cx2 = 0.0f, Cy2 = 0.0f;
 #pragma unroll
         for (int ox = 0; ox < 3; ++ox) {
-            float T[3] = {0.0f, 0.0f, 0.0f}, Ty[3] = {0.0f, 0.0f, 0.0f}, Tz[3] = {0.0f, 0.0f, 0.0f};
+            float2 T01 = zero, Ty01 = zero, Tz01 = zero, TTz2 = zero;
+            float Ty2 = 0.0f;
 #pragma unroll
             for (int oy = 0; oy < 3; ++oy) {
-                float Z0[3] = {0.0f, 0.0f, 0.0f}, Zd[3] = {0.0f, 0.0f, 0.0f};
+                float2 Z01 = zero, Zd01 = zero, ZZd2 = zero;
 #pragma unroll
                 for (int oz = 0; oz < 3; ++oz) {
-                    const int node = NX[ox] + NY[oy] + NZ[oz];
-                    const float4 g = TILE ? sq[node] : __ldg(&gvel[node]);
+                    const int node = TILE ? NX[ox] + NY[oy] + oz : NX[ox] + NY[oy] + NZ[oz];
+                    float4 g = TILE ? sq[node] : __ldg(&gvel[node]);
+                    if (!TILE) g.w = g.z;
                     const float wz = q.w[oz][2], wd = wzd[oz];
-                    Z0[0] += wz * g.x; Z0[1] += wz * g.y; Z0[2] += wz * g.z;
-                    Zd[0] += wd * g.x; Zd[1] += wd * g.y; Zd[2] += wd * g.z;
+                    Z01 = fma2(bc2(wz), make_float2(g.x, g.y), Z01);
+                    Zd01 = fma2(bc2(wd), make_float2(g.x, g.y), Zd01);
+                    ZZd2 = fma2(make_float2(wz, wd), make_float2(g.z, g.w), ZZd2);
                 }
-                const float wy = q.w[oy][1], wd = wyd[oy];
-#pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    T[i] += wy * Z0[i];
-                    Ty[i] += wd * Z0[i];
-                    Tz[i] += wy * Zd[i];
-                }
+                const float2 wy = bc2(q.w[oy][1]), wd = bc2(wyd[oy]);
+                T01 = fma2(wy, Z01, T01);
+                Ty01 = fma2(wd, Z01, Ty01);
+                Tz01 = fma2(wy, Zd01, Tz01);
+                TTz2 = fma2(wy, ZZd2, TTz2);
+                Ty2 += wyd[oy] * ZZd2.x;
             }
-            const float wx = q.w[ox][0], wd = wxd[ox];
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                nv[i] += wx * T[i];
-                nC[3 * i] += wd * T[i];
-                nC[3 * i + 1] += wx * Ty[i];
-                nC[3 * i + 2] += wx * Tz[i];
-            }
+            const float2 wx = bc2(q.w[ox][0]), wd = bc2(wxd[ox]);
+            v01 = fma2(wx, T01, v01);
+            Cx01 = fma2(wd, T01, Cx01);
+            Cy01 = fma2(wx, Ty01, Cy01);
+            Cz01 = fma2(wx, Tz01, Cz01);
+            v2Cz2 = fma2(wx, TTz2, v2Cz2);
+            Cx2 += wxd[ox] * TTz2.x;
+            Cy2 += q.w[ox][0] * Ty2;
         }
+        nv[0] = v01.x; nv[1] = v01.y; nv[2] = v2Cz2.x;
+        nC[0] = Cx01.x; nC[1] = Cy01.x; nC[2] = Cz01.x;
+        nC[3] = Cx01.y; nC[4] = Cy01.y; nC[5] = Cz01.y;
+        nC[6] = Cx2;    nC[7] = Cy2;    nC[8] = v2Cz2.y;
         const float cfac = (float)(4.0 * prm.inv_dx * prm.inv_dx);
 #pragma unroll
         for (int k = 0; k < 9; ++k) nC[k] *= cfac;
@@ -444,7 +457,9 @@ __global__ void __launch_bounds__(kG2PThreads, MINB) k_g2p(const SC scn, const P
         for (int i = tid; i < qn; i += kG2PThreads) {
             const int ix = fdiv(i, qyz), r = i - ix * qyz.d, iy = fdiv(r, qz);
             const int gx = lo[0] + ix, gy = lo[1] + iy, gz = lo[2] + r - iy * qz.d;
-            sq[i] = gvel[((long long)gx * ng + gy) * ng + gz];
+            float4 g = gvel[((long long)gx * ng + gy) * ng + gz];
+            g.w = g.z;
+            sq[i] = g;
         }
         const FastDiv cyz = make_fastdiv(cd[1] * cd[2]), cz = make_fastdiv(cd[2]);
         for (int i = tid; i < cn; i += kG2PThreads) {
