@@ -1033,6 +1033,11 @@ constexpr int kAC = 1024;   // staged cubic nodes per CTA (16 B each)
 
 // Gathers of k_adj_particle for one particle, from the CTA's shared-memory
 // tile (TILE) or from global memory with the reference's clamped indices.
+// Both are folded over z, then y, then x, sums that share a weight or a value in
+// packed pairs (b.w holds b.z again in the tile): 1M particles 316 us with the
+// x and y weights multiplied out per row, 299 now.  The kernel is bound by latency
+// at 16 warps per SM (45% of issue slots): with 3 CTAs per SM, without spills, the
+// backward of 8 substeps took 370 us longer, with 5 as long.
 template <bool TILE>
 __device__ __forceinline__ void adj_gather(const float xp[3], float inv_dx, float dx, float K, int ng,
                                            const float vt[3], const float Ct[9], const float mv[3], float m,
@@ -1056,99 +1061,126 @@ __device__ __forceinline__ void adj_gather(const float xp[3], float inv_dx, floa
             DY[o] = ((float)o - q.fx[1]) * dx;
             DZ[o] = ((float)o - q.fx[2]) * dx;
         }
-        float z0[3] = {0.0f, 0.0f, 0.0f}, z1[3] = {0.0f, 0.0f, 0.0f};   // per axis of xbar
+        const float2 zero = make_float2(0.0f, 0.0f);
+        // components x and y in packed pairs, z with its dpos_z moment
+        const float2 C0 = make_float2(K * Ct[0], K * Ct[3]), C1 = make_float2(K * Ct[1], K * Ct[4]),
+                     C2 = make_float2(K * Ct[2], K * Ct[5]);
+        const float2 a0 = make_float2(aff[0], aff[3]), a1 = make_float2(aff[1], aff[4]), a2 = make_float2(aff[2], aff[5]);
+        const float C20 = K * Ct[6], C21 = K * Ct[7], C22 = K * Ct[8];
+        float2 vs01 = zero, mv01 = zero, ax01 = zero, ay01 = zero, az01 = zero, mvaz2 = zero;
+        float vs2 = 0.0f, ax2 = 0.0f, ay2 = 0.0f;
+        float z0[2] = {0.0f, 0.0f}, z1 = 0.0f;   // per axis of xbar
 #pragma unroll
         for (int ox = 0; ox < 3; ++ox) {
-            float ux[3], cx[3];
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                ux[i] = vt[i] + K * Ct[3 * i] * DX[ox];
-                cx[i] = mv[i] + aff[3 * i] * DX[ox];
-            }
+            const float2 ux01 = fma2(C0, bc2(DX[ox]), make_float2(vt[0], vt[1]));
+            const float2 cx01 = fma2(a0, bc2(DX[ox]), make_float2(mv[0], mv[1]));
+            const float ux2 = vt[2] + C20 * DX[ox], cx2 = mv[2] + aff[6] * DX[ox];
 #pragma unroll
             for (int oy = 0; oy < 3; ++oy) {
-                float uxy[3], cxy[3];
-#pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    uxy[i] = ux[i] + K * Ct[3 * i + 1] * DY[oy];
-                    cxy[i] = cx[i] + aff[3 * i + 1] * DY[oy];
-                }
-                float Z0 = 0.0f, Z1 = 0.0f, Gz[3] = {0.0f, 0.0f, 0.0f}, Az[3] = {0.0f, 0.0f, 0.0f},
-                      Azd[3] = {0.0f, 0.0f, 0.0f};
+                const float2 uxy01 = fma2(C1, bc2(DY[oy]), ux01), cxy01 = fma2(a1, bc2(DY[oy]), cx01);
+                const float uxy2 = ux2 + C21 * DY[oy], cxy2 = cx2 + aff[7] * DY[oy];
+                float2 Z = zero, G01 = zero, A01 = zero, Ad01 = zero, AAd2 = zero;   // Z: (Z0, Z1); AAd2: (Az, Azd).z
+                float G2 = 0.0f;
+                const int row = TILE ? ((q.b[0] + ox - lo[0]) * qd[1] + (q.b[1] + oy - lo[1])) * qd[2] + q.b[2] - lo[2] : 0;
 #pragma unroll
                 for (int oz = 0; oz < 3; ++oz) {
                     float4 g, an;
                     if (TILE) {
-                        const int t = ((q.b[0] + ox - lo[0]) * qd[1] + (q.b[1] + oy - lo[1])) * qd[2] + q.b[2] + oz - lo[2];
-                        g = sv[t];
-                        an = sa[t];
+                        g = sv[row + oz];
+                        an = sa[row + oz];
                     } else {
                         const int node = node_of(q.b[0] + ox, q.b[1] + oy, q.b[2] + oz, ng);
                         g = __ldg(&gvel[node]);
                         an = __ldg(&A[node]);
                     }
-                    const float u0 = uxy[0] + K * Ct[2] * DZ[oz], u1 = uxy[1] + K * Ct[5] * DZ[oz],
-                                u2 = uxy[2] + K * Ct[8] * DZ[oz];
-                    const float c0 = cxy[0] + aff[2] * DZ[oz], c1 = cxy[1] + aff[5] * DZ[oz],
-                                c2 = cxy[2] + aff[8] * DZ[oz];
-                    const float wbar = (g.x * u0 + g.y * u1 + g.z * u2) + (an.x * c0 + an.y * c1 + an.z * c2) + an.w * m;
+                    const float2 g01 = make_float2(g.x, g.y), an01 = make_float2(an.x, an.y);
+                    const float2 u01 = fma2(C2, bc2(DZ[oz]), uxy01), c01 = fma2(a2, bc2(DZ[oz]), cxy01);
+                    const float u2 = uxy2 + C22 * DZ[oz], c2 = cxy2 + aff[8] * DZ[oz];
+                    const float2 t = fma2(an01, c01, mul2(g01, u01));
+                    const float wbar = (t.x + t.y) + (g.z * u2 + (an.z * c2 + an.w * m));
                     const float wz = q.w[oz][2], wzd = wz * DZ[oz];
-                    Z0 += wz * wbar;
-                    Z1 += q.dw[oz][2] * wbar;
-                    Gz[0] += wz * g.x; Gz[1] += wz * g.y; Gz[2] += wz * g.z;
-                    Az[0] += wz * an.x; Az[1] += wz * an.y; Az[2] += wz * an.z;
-                    Azd[0] += wzd * an.x; Azd[1] += wzd * an.y; Azd[2] += wzd * an.z;
+                    Z = fma2(make_float2(wz, q.dw[oz][2]), bc2(wbar), Z);
+                    G01 = fma2(bc2(wz), g01, G01);
+                    G2 += wz * g.z;
+                    A01 = fma2(bc2(wz), an01, A01);
+                    Ad01 = fma2(bc2(wzd), an01, Ad01);
+                    AAd2 = fma2(make_float2(wz, wzd), bc2(an.z), AAd2);
                 }
                 const float wx = q.w[ox][0], wy = q.w[oy][1], wxy = wx * wy;
-                z0[0] += q.dw[ox][0] * wy * Z0;
-                z0[1] += wx * q.dw[oy][1] * Z0;
-                z1[2] += wxy * Z1;
+                z0[0] += q.dw[ox][0] * wy * Z.x;
+                z0[1] += wx * q.dw[oy][1] * Z.x;
+                z1 += wxy * Z.y;
                 const float wxyx = wxy * DX[ox], wxyy = wxy * DY[oy];
-#pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    vsum[i] += wxy * Gz[i];
-                    mvb[i] += wxy * Az[i];
-                    affb[3 * i] += wxyx * Az[i];
-                    affb[3 * i + 1] += wxyy * Az[i];
-                    affb[3 * i + 2] += wxy * Azd[i];
-                }
+                const float2 w2 = bc2(wxy);
+                vs01 = fma2(w2, G01, vs01);
+                vs2 += wxy * G2;
+                mv01 = fma2(w2, A01, mv01);
+                ax01 = fma2(bc2(wxyx), A01, ax01);
+                ay01 = fma2(bc2(wxyy), A01, ay01);
+                az01 = fma2(w2, Ad01, az01);
+                mvaz2 = fma2(w2, AAd2, mvaz2);
+                ax2 += wxyx * AAd2.x;
+                ay2 += wxyy * AAd2.x;
             }
         }
+        vsum[0] = vs01.x; vsum[1] = vs01.y; vsum[2] = vs2;
+        mvb[0] = mv01.x;  mvb[1] = mv01.y;  mvb[2] = mvaz2.x;
+        affb[0] = ax01.x; affb[1] = ay01.x; affb[2] = az01.x;
+        affb[3] = ax01.y; affb[4] = ay01.y; affb[5] = az01.y;
+        affb[6] = ax2;    affb[7] = ay2;    affb[8] = mvaz2.y;
         xb[0] += inv_dx * z0[0];
         xb[1] += inv_dx * z0[1];
-        xb[2] += inv_dx * z1[2];
+        xb[2] += inv_dx * z1;
     }
     {
         CubicD cw;
         cubic_weights_d(xp, inv_dx, ng, cw);
+        // Per node: wbar = b.x d1 + b.y, and b.z for the Laplacian's position part.
+        // Folded over z, then y, then x, in packed pairs where two sums share a
+        // weight or a value.
         float dsum = 0.0f;
+        float x0 = 0.0f, x1 = 0.0f, x2 = 0.0f;
+        const float2 zero = make_float2(0.0f, 0.0f);
 #pragma unroll
-        for (int ox = 0; ox < 4; ++ox)
+        for (int ox = 0; ox < 4; ++ox) {
+            // sums over y: wy (swd, swb); wy (g0, g2); w2y (g0, g2) + wy (g1, g3); dwy swb; wy sdwb; dwy g0; dw2y g0 + dwy g1
+            float2 W = zero, G = zero, GS = zero;
+            float dW = 0.0f, wD = 0.0f, dG = 0.0f, tG = 0.0f;
 #pragma unroll
             for (int oy = 0; oy < 4; ++oy) {
-                const int row = TILE ? ((cw.b[0] + ox - lo[0] + 1) * cd[1] + (cw.b[1] + oy - lo[1] + 1)) * cd[2]
+                const int row = TILE ? ((cw.b[0] + ox - lo[0] + 1) * cd[1] + (cw.b[1] + oy - lo[1] + 1)) * cd[2] +
+                                           cw.b[2] - lo[2] + 1
                                      : (clampi(cw.b[0] + ox, 0, ng - 1) * ng + clampi(cw.b[1] + oy, 0, ng - 1)) * ng;
-                float swd = 0.0f, swb = 0.0f, sdwb = 0.0f, g0 = 0.0f, g1 = 0.0f, g2 = 0.0f, g3 = 0.0f;
+                float2 sw = zero, g02 = zero, g13 = zero;   // sums over z: w (b.x, wbar); (w, dw) b.z; (w2, dw2) b.z
+                float sdwb = 0.0f;
 #pragma unroll
                 for (int oz = 0; oz < 4; ++oz) {
-                    const float4 bn = TILE ? sb[row + cw.b[2] + oz - lo[2] + 1] : __ldg(&B[row + clampi(cw.b[2] + oz, 0, ng - 1)]);
-                    const float wz = cw.w[oz][2], dwz = cw.dw[oz][2];
+                    const float4 bn = TILE ? sb[row + oz] : __ldg(&B[row + clampi(cw.b[2] + oz, 0, ng - 1)]);
                     const float wbar = bn.x * d1 + bn.y;
-                    swd += wz * bn.x;
-                    swb += wz * wbar;
-                    sdwb += dwz * wbar;
-                    g0 += wz * bn.z;
-                    g1 += cw.w2[oz][2] * bn.z;
-                    g2 += dwz * bn.z;
-                    g3 += cw.dw2[oz][2] * bn.z;
+                    const float2 zz = make_float2(bn.z, TILE ? bn.w : bn.z);
+                    sw = fma2(bc2(cw.w[oz][2]), make_float2(bn.x, wbar), sw);
+                    sdwb += cw.dw[oz][2] * wbar;
+                    g02 = fma2(make_float2(cw.w[oz][2], cw.dw[oz][2]), zz, g02);
+                    g13 = fma2(make_float2(cw.w2[oz][2], cw.dw2[oz][2]), zz, g13);
                 }
-                const float wx = cw.w[ox][0], wy = cw.w[oy][1], dwx = cw.dw[ox][0], dwy = cw.dw[oy][1];
-                const float sx = cw.w2[ox][0], sy = cw.w2[oy][1], tx = cw.dw2[ox][0], ty = cw.dw2[oy][1];
-                dsum += wx * wy * swd;
-                xb[0] += inv_dx * dwx * wy * swb + lb * ((tx * wy + dwx * sy) * g0 + dwx * wy * g1);
-                xb[1] += inv_dx * wx * dwy * swb + lb * ((sx * dwy + wx * ty) * g0 + wx * dwy * g1);
-                xb[2] += inv_dx * wx * wy * sdwb + lb * ((sx * wy + wx * sy) * g2 + wx * wy * g3);
+                const float wy = cw.w[oy][1], dwy = cw.dw[oy][1];
+                W = fma2(bc2(wy), sw, W);
+                G = fma2(bc2(wy), g02, G);
+                GS = fma2(bc2(cw.w2[oy][1]), g02, fma2(bc2(wy), g13, GS));
+                dW += dwy * sw.y;
+                wD += wy * sdwb;
+                dG += dwy * g02.x;
+                tG += cw.dw2[oy][1] * g02.x + dwy * g13.x;
             }
+            const float wx = cw.w[ox][0], dwx = cw.dw[ox][0], sx = cw.w2[ox][0], tx = cw.dw2[ox][0];
+            dsum += wx * W.x;
+            x0 += inv_dx * dwx * W.y + lb * (tx * G.x + dwx * GS.x);
+            x1 += inv_dx * wx * dW + lb * (sx * dG + wx * tG);
+            x2 += inv_dx * wx * wD + lb * (sx * G.y + wx * GS.y);
+        }
+        xb[0] += x0;
+        xb[1] += x1;
+        xb[2] += x2;
         d1b += dsum;
     }
 }
@@ -1223,7 +1255,9 @@ __global__ void __launch_bounds__(128, 4) k_adj_particle(const pm_params prm, co
         for (int i = tid; i < cn; i += blockDim.x) {
             const int ix = fdiv(i, cyz), r = i - ix * cyz.d, iy = fdiv(r, cz);
             const int gx = lo[0] - 1 + ix, gy = lo[1] - 1 + iy, gz = lo[2] - 1 + r - iy * cz.d;
-            sb[i] = B[((long long)gx * ng + gy) * ng + gz];
+            float4 b = B[((long long)gx * ng + gy) * ng + gz];
+            b.w = b.z;                       // a packed operand
+            sb[i] = b;
         }
     }
     __syncthreads();
@@ -1283,9 +1317,7 @@ __global__ void __launch_bounds__(128, 4) k_adj_particle(const pm_params prm, co
     for (int k = 0; k < 9; ++k) aff[k] = taff[k * taff_stride + p];
     // ---- gathers (quadratic: G2P adjoint position part and P2G adjoint;
     // cubic: damage scatter adjoint and the Laplacian's position part)
-    float vsum[3] = {0.0f, 0.0f, 0.0f}, mvb[3] = {0.0f, 0.0f, 0.0f}, affb[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) affb[k] = 0.0f;
+    float vsum[3], mvb[3], affb[9];
     float d1b = ain.d[p];
     {
         const float d1 = post.d[p];

@@ -777,6 +777,9 @@ __device__ __forceinline__ void red_fix(long long *addr, float v, float scale) {
     if (q != 0) atomicAdd((unsigned long long *)addr, (unsigned long long)q);
 }
 
+// Brings the line to L2 while the caller does something else.
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 __device__ __forceinline__ unsigned lanemask_lt() {
     unsigned m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));

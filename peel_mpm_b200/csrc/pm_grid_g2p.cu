@@ -428,6 +428,11 @@ __global__ void __launch_bounds__(kG2PThreads, MINB) k_g2p(const SC scn, const P
             qb[a] = reg ? (int)fb : 0;
         }
     }
+    if (valid) {   // read after the gathers: 71 us without, 67 with, 1M particles
+        const float *Fin = prm.use_f_clamp ? P.Fo : P.F;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) prefetch_l2(&Fin[k * ps + p]);
+    }
     // bounding box of the regular particles' base cells
     int cl[3], ch[3];
 #pragma unroll
