@@ -80,13 +80,13 @@ BYTES_PER_NODE = 80
 # `traffic` and its issue-bound floor (warp instructions / (4 schedulers x
 # SMs x SM clock)).
 NCU_KERNELS = {
-    "k_count": {"dram_bytes": None, "warp_inst": None},
-    "k_offsets": {"dram_bytes": None, "warp_inst": None},
-    "k_place": {"dram_bytes": None, "warp_inst": None},
-    "k_rank": {"dram_bytes": None, "warp_inst": None},
-    "k_stress": {"dram_bytes": None, "warp_inst": None},
-    "k_p2g_sweep": {"dram_bytes": None, "warp_inst": None},
-    "k_g2p": {"dram_bytes": 54698240 + 46928640, "warp_inst": 53436416},
+    "k_count": {"dram_bytes": 14887168, "warp_inst": 4003004},
+    "k_offsets": {"dram_bytes": 1429760, "warp_inst": 482551},
+    "k_place": {"dram_bytes": 18054400, "warp_inst": 3670016},
+    "k_rank": {"dram_bytes": 5716480, "warp_inst": 5091289},
+    "k_stress": {"dram_bytes": 195964928 + 51072768, "warp_inst": 39837552},
+    "k_p2g_sweep": {"dram_bytes": 81618176 + 1478656, "warp_inst": 66801624},
+    "k_g2p": {"dram_bytes": 54691328 + 45396480, "warp_inst": 48168960},
 }
 P2G_KERNELS = ("k_count", "k_offsets", "k_place", "k_rank", "k_stress", "k_p2g_sweep")
 LAUNCHES_PER_SUBSTEP = 3 + len(P2G_KERNELS)   # and clock, grid, g2p; one scene or a batch of any number
