@@ -332,7 +332,7 @@ __device__ __forceinline__ void pix_add(PixAcc &p, const float4 &A, const float4
     const int rd = __float_as_int(Cc.w);
     if (abs(px - __float_as_int(B.z)) > rd || abs(py - __float_as_int(B.w)) > rd) return;
     const float dx = ((float)px + 0.5f) - A.x, dy = ((float)py + 0.5f) - A.y;
-    const float power = -0.5f * (A.z * dx * dx + B.x * dy * dy) - A.w * dx * dy;
+    const float power = fmaf(-0.5f, fmaf(A.z * dx, dx, __fmul_rn(B.x * dy, dy)), -__fmul_rn(A.w * dx, dy));
     if (power < -6.0f) return;
     const float ga = __expf(power < 0.0f ? power : 0.0f);
     if (!(ga > (1.0f / 255.0f))) return;
@@ -503,8 +503,8 @@ __device__ __forceinline__ bool draw_part(const pm_camera &cam, const pm_render_
             const float4 A = sh.a[j], B = sh.b[j], C = sh.c[j], D = sh.d[j];
             const float dx = pxc - A.x;
             const float2 dy = make_float2(pyc0 - A.y, pyc1 - A.y);
-            // power as in pix_add, with its roundings: the same pixels pass
-            const float2 q = fma2(mul2(make_float2(C.x, C.y), dy), dy, bc2(A.z * dx * dx));
+            // power with pix_add's roundings, operation by operation: the same pixels pass 1/255
+            const float2 q = fma2(bc2(A.z * dx), bc2(dx), mul2(mul2(make_float2(C.x, C.y), dy), dy));
             const float2 power = fma2(bc2(-0.5f), q, mul2(bc2(-(A.w * dx)), dy));
             const float2 p2 = mul2(make_float2(fminf(power.x, 0.0f), fminf(power.y, 0.0f)), bc2(kLog2e));
             float2 ga = make_float2(ex2(p2.x), ex2(p2.y));
