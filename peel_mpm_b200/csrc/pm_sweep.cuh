@@ -25,6 +25,11 @@
 // added to the plane) at every 256th particle of the cell's 4^3-cell sub-block in
 // Morton order of its cells.  The sums of a substep are thus fixed by the
 // particles alone, not by the order of arrival, the launch or the batch.
+//
+// Bound by instruction issue (64%) and the FMA pipe.  1M displaced particles, 6 to
+// 11 per cell: 133 us, the former tile kernel 129.  It gains where cells hold more
+// or units are few: with the counted binning 8.8M particles at 27 per cell go from
+// 6,360 to 5,250 us per two substeps, 138k from 1,227 to 597 us per six.
 #pragma once
 
 #include "pm_common.cuh"
