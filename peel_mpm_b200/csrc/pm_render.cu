@@ -474,7 +474,8 @@ __device__ __forceinline__ bool draw_part(const pm_camera &cam, const pm_render_
             zfar = fmaxf(zfar, __uint_as_float(__reduce_max_sync(all, keep ? __float_as_uint(z) : 0u)));
             if (!((zfar - zn) * inv_tau <= kMaxRange)) return false;
             if (zn < zref) {
-                const float sc = ex2(-(zref - zn) * tau2);   // 0 the first time
+                // nothing to rescale the first time (and infinity times 1 / tau = 0, tau infinite, is not a number)
+                const float sc = zref < inf ? ex2(-(zref - zn) * tau2) : 0.0f;
                 const float2 sc2 = bc2(sc);
                 c0 = mul2(c0, sc2);
                 c1 = mul2(c1, sc2);
