@@ -189,12 +189,14 @@ int pm_p2g(const pm_params *prm, const pm_particles *P, void *ws, size_t ws_byte
     if ((rc = check_device()) || (rc = check_params(prm)) || (rc = check_particles(P, true))) return rc;
     pm::WS w;
     if ((rc = get_ws(ws, ws_bytes, P->n, prm->n_grid, &w))) return rc;
-    // a piece by itself starts clean, whether or not a clock or a grid update ran since the last one: marks left
-    // over would keep blocks off the new list, counters left over would move the payload's runs
-    cudaMemsetAsync(w.block_mask, 0, (size_t)w.n_blocks, (cudaStream_t)stream);
-    cudaMemsetAsync(&w.ctrl->n_work, 0, 4 * sizeof(unsigned), (cudaStream_t)stream);
-    pm::launch_p2g(pm::PlainScenes{*prm}, pm::make_parts(P), w, (cudaStream_t)stream, -1, prm->p2g_ctas_per_sm,
-                   prm->stress_ctas_per_sm);
+    cudaStream_t s = (cudaStream_t)stream;
+    // Counters left over from a P2G without a clock since would list blocks twice and move the payload's runs.
+    cudaMemsetAsync(&w.ctrl->n_active, 0, sizeof(unsigned), s);
+    cudaMemsetAsync(&w.ctrl->n_work, 0, 4 * sizeof(unsigned), s);
+    pm::launch_p2g(pm::PlainScenes{*prm}, pm::make_parts(P), w, s, -1, prm->p2g_ctas_per_sm, prm->stress_ctas_per_sm);
+    // The touched blocks are on the list.  The grid update unmarks them too, but it need not follow, and a mark that
+    // stays keeps its block off every later list.
+    cudaMemsetAsync(w.block_mask, 0, (size_t)w.n_blocks, s);
     return cuda_check("pm_p2g");
 }
 
