@@ -458,6 +458,9 @@ __device__ __forceinline__ FixScale fix_scale(unsigned bound_bits) {
     return f;
 }
 __device__ __forceinline__ long long to_fix(float v, float scale) { return __float2ll_rn(v * scale); }
+__device__ __forceinline__ long long fix_add(long long a, long long b) {   // modulo 2^64
+    return (long long)((unsigned long long)a + (unsigned long long)b);
+}
 __device__ __forceinline__ float from_fix(long long q, float unit) { return __ll2float_rn(q) * unit; }
 // Magnitude bound of a value for the control block's atomicMax (NaN counts as 0).
 __device__ __forceinline__ unsigned bound_bits(float v) {

@@ -159,7 +159,7 @@ __device__ __forceinline__ void plane_words_add(char *at, int stride, const long
 #pragma unroll
     for (int k = 0; k < NC; ++k) o[k] = *(long long *)(at + k * stride);
 #pragma unroll
-    for (int k = 0; k < NC; ++k) *(long long *)(at + k * stride) = o[k] + q[k];
+    for (int k = 0; k < NC; ++k) *(long long *)(at + k * stride) = fix_add(o[k], q[k]);
     __syncwarp();
 }
 constexpr int kOddRow = 64, kRowBytes = 8 * kPlaneCols;   // rows an odd number apart: xor kOddRow (see plane_word)
@@ -168,7 +168,11 @@ __device__ __forceinline__ void red_add(long long *g, long long q) {   // g: glo
     asm volatile("red.global.add.u64 [%0], %1;" ::"l"(__cvta_generic_to_global(g)), "l"(q) : "memory");
 }
 // Sends a plane's nonzero words to the global sums (node (r, c) at
-// gp + gs (r ng + c)) and clears them.
+// gp + gs (r ng + c)) and clears them.  A float sum that is not a number or
+// infinite was converted to +-2^63 or 2^63 - 1 and has wrapped the word's top
+// bit: without that bit (a unit's finite sums stay below 2^62, see
+// kDenseSubblock) it counts for nothing, so that a particle gone astray does not
+// throw its neighbours about.
 template <int NC, int ROWS, int COLS, int NP>
 __device__ __forceinline__ void plane_out(long long (&pl)[NP][ROWS * kPlaneCols], long long *gp, int gs, long long ng,
                                           int lane) {
@@ -177,10 +181,11 @@ __device__ __forceinline__ void plane_out(long long (&pl)[NP][ROWS * kPlaneCols]
         long long *g = gp + gs * (r * ng + c);
 #pragma unroll
         for (int k = 0; k < NC; ++k) {
-            const long long q = pl[k][i];
-            if (q != 0) {
+            const long long v = pl[k][i];
+            if (v != 0) {
                 pl[k][i] = 0;
-                red_add(g + k, q);
+                const long long q = (long long)((unsigned long long)v << 1) >> 1;
+                if (q != 0) red_add(g + k, q);
             }
         }
     }
@@ -279,7 +284,7 @@ struct QuadSums {
             to_q(sh, sp[2 * lane], sp[2 * lane + 1], q);
             const int i = plane_word((l >> 3) + lane / 3, (l & 7) + lane % 3);
 #pragma unroll
-            for (int k = 0; k < NC; ++k) sh.qpl[wid][k][i] += q[k];
+            for (int k = 0; k < NC; ++k) sh.qpl[wid][k][i] = fix_add(sh.qpl[wid][k][i], q[k]);
         }
         __syncwarp();
     }
@@ -342,8 +347,9 @@ struct CubicSums {
         if (lane < 25) {
             const float2 v = sp[lane];
             const int i = plane_word((l >> 3) + lane / 5, (l & 7) + lane % 5);
-            sh.cpl[wid - kSweepQ][0][i] += to_fix(v.x, sh.scale[2]);
-            sh.cpl[wid - kSweepQ][1][i] += to_fix(v.y, sh.scale[3]);
+            long long(&pl)[2][kCRows * kPlaneCols] = sh.cpl[wid - kSweepQ];
+            pl[0][i] = fix_add(pl[0][i], to_fix(v.x, sh.scale[2]));
+            pl[1][i] = fix_add(pl[1][i], to_fix(v.y, sh.scale[3]));
         }
         __syncwarp();
     }
@@ -416,8 +422,10 @@ struct CubicLapSums {
             clear();
         }
         __syncwarp();
-        if (lane < 25)
-            sh.cpl[wid - kSweepQ][0][plane_word((l >> 3) + lane / 5, (l & 7) + lane % 5)] += to_fix(sp[lane], sh.scale[2]);
+        if (lane < 25) {
+            long long &at = sh.cpl[wid - kSweepQ][0][plane_word((l >> 3) + lane / 5, (l & 7) + lane % 5)];
+            at = fix_add(at, to_fix(sp[lane], sh.scale[2]));
+        }
         __syncwarp();
     }
     __device__ __forceinline__ void out(SweepShared &sh, int wid, int lane, int X) {
