@@ -45,7 +45,7 @@ struct TapeHead {
     long long step;
     double time;
     unsigned n_work;    // non-empty units of the substep
-    unsigned pad;
+    unsigned n_clamped; // of these, the ones with cells that need clamped nodes
     float col_origin[PM_MAX_COLLIDERS][3];   // the substep's collider origins and velocities
     float col_vel[PM_MAX_COLLIDERS][3];
 };
@@ -241,58 +241,10 @@ __global__ void __launch_bounds__(256) k_adj_pre(const pm_params prm, const Part
     }
 }
 
-// One particle whose stencil needs the reference's edge clamping, straight
-// into the global adjoint grid (4 int64 per node: momentum adjoint, damage
-// adjoint).
-__device__ __noinline__ void adj_scatter_global(const float xp[3], const float vt[3], const float kc[9], float lb,
-                                                float inv_dx, float dx, int ng, float smom, float slap,
-                                                long long *acc) {
-    Quad q;
-    quad_weights(xp, inv_dx, ng, q);
-    Cubic c;
-    cubic_weights(xp, inv_dx, ng, c);
-    float wq[3][4], U[3][4][3];
-#pragma unroll
-    for (int ax = 0; ax < 3; ++ax) {
-        const bool s1 = q.b[ax] != c.b[ax];   // quadratic base one node above the cubic one
-#pragma unroll
-        for (int o = 0; o < 4; ++o) {
-            float w = 0.0f, oq = 0.0f;
-            if (s1) {
-                if (o >= 1) { w = q.w[o - 1][ax]; oq = (float)(o - 1); }
-            } else {
-                if (o < 3) { w = q.w[o][ax]; oq = (float)o; }
-            }
-            wq[ax][o] = w;
-            const float dp = (oq - q.fx[ax]) * dx;
-#pragma unroll
-            for (int i = 0; i < 3; ++i) U[ax][o][i] = kc[3 * i + ax] * dp;
-        }
-    }
-#pragma unroll
-    for (int ox = 0; ox < 4; ++ox)
-#pragma unroll
-        for (int oy = 0; oy < 4; ++oy) {
-            const float ab = lb * (c.w2[ox][0] * c.w[oy][1] + c.w[ox][0] * c.w2[oy][1]);
-            const float e = lb * (c.w[ox][0] * c.w[oy][1]);
-            const float wxy = wq[0][ox] * wq[1][oy];
-            const float b0 = vt[0] + U[0][ox][0] + U[1][oy][0];
-            const float b1 = vt[1] + U[0][ox][1] + U[1][oy][1];
-            const float b2 = vt[2] + U[0][ox][2] + U[1][oy][2];
-            const long long row = ((long long)clampi(c.b[0] + ox, 0, ng - 1) * ng + clampi(c.b[1] + oy, 0, ng - 1)) * ng;
-#pragma unroll
-            for (int oz = 0; oz < 4; ++oz) {
-                const float wk = wxy * wq[2][oz];
-                long long *g = acc + 4 * (row + clampi(c.b[2] + oz, 0, ng - 1));
-                red_fix(g, wk * (b0 + U[2][oz][0]), smom);
-                red_fix(g + 1, wk * (b1 + U[2][oz][1]), smom);
-                red_fix(g + 2, wk * (b2 + U[2][oz][2]), smom);
-                red_fix(g + 3, ab * c.w[oz][2] + e * c.w2[oz][2], slap);
-            }
-        }
-}
-
 // ---------------------------------------------------------------- k_adj_sweep
+struct NoMark {
+    static __device__ __forceinline__ void node(const SweepShared &, const WS *, int, int, int) {}
+};
 // The G2P adjoint scatter over the forward substep's non-empty units, with the
 // forward P2G's sweep (pm_sweep.cuh): quadratic planes sum w (vt + K Ct dpos)
 // into the momentum adjoint, cubic planes lb W'' into the damage adjoint, int64
@@ -300,6 +252,7 @@ __device__ __noinline__ void adj_scatter_global(const float xp[3], const float v
 // so no block marks are needed.
 __global__ void __launch_bounds__(kSweepThreads, 3) k_adj_sweep(const __grid_constant__ pm_params prm,
                                                                 const int *__restrict__ work,
+                                                                const int *__restrict__ clamped,
                                                                 const int2 *__restrict__ cells,
                                                                 const unsigned char *__restrict__ split,
                                                                 const TapeHead *head,
@@ -331,18 +284,12 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_adj_sweep(const __grid_con
     while (now.x >= 0) {
         const int i = now.x, u = work[i], x0 = now.y & 255, x1 = now.y >> 8;
         const unsigned blk = (unsigned)u / kBlockUnits;
-        const int org[3] = {(int)(blk / ((unsigned)nb * nb)) * kSortBlock + ((u >> 1) & 1) * kUnitX,
-                            (int)(blk / nb % nb) * kSortBlock + (u & 1) * kUnitY, (int)(blk % nb) * kSortBlock};
-        bool edge = false;                // particles that need clamped nodes
-        int2 cell = make_int2(0, 0);
+        int org[3];
+        unit_origin(u, blk, nb, org);
         if (wid >= x0 && wid < x1) {
-            cell = cells[(long long)i * kUnitCells + tid];
-            const int c[3] = {tid >> 5, (tid >> 3) & 3, tid & 7};
-            bool reg = true;
-#pragma unroll
-            for (int a = 0; a < 3; ++a) reg = reg && org[a] + c[a] >= 1 && org[a] + c[a] <= ng - 4;
-            edge = cell.y > 0 && !reg;
-            const int cnt = reg ? cell.y : 0;
+            const int2 cell = cells[(long long)i * kUnitCells + tid];
+            const int g[3] = {org[0] + (tid >> 5), org[1] + ((tid >> 3) & 3), org[2] + (tid & 7)};
+            const int cnt = clamped_cell(g, ng) ? 0 : cell.y;
             sh.cell[tid] = make_int2(cell.x, cnt);
             sh.split[tid] = split[(long long)i * kUnitCells + tid];
             const int rows = __reduce_max_sync(0xffffffffu, cnt);
@@ -354,24 +301,9 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_adj_sweep(const __grid_con
             sh.g_quad = acc + 4 * (((long long)org[0] * ng + org[1]) * ng + org[2]);
             sh.g_cubic = acc + 4 * (((long long)(org[0] - 1) * ng + org[1] - 1) * ng + org[2] - 1) + 3;
         }
-        const bool edges = __syncthreads_or(edge);
+        __syncthreads();
         unsigned take = 0;                // the next item is taken while this one is swept
         if (tid == kSweepThreads - 1) take = gridDim.x + atomicAdd(&actl->work_next, 1u);
-        if (edges) {                      // the cell's particles over the lanes of its warp
-            const unsigned eb = __ballot_sync(0xffffffffu, edge);
-            for (unsigned m = eb; m; m &= m - 1) {
-                const int l = __ffs(m) - 1;
-                const int f = __shfl_sync(0xffffffffu, cell.x, l), cnt = __shfl_sync(0xffffffffu, cell.y, l);
-                for (int k = lane; k < cnt; k += 32) {
-                    const long long s = place_of(f, k);
-                    const float4 *p = (const float4 *)pay_at(pay, s);
-                    const float4 p0 = p[0], p1 = p[32], p2 = p[64], p3 = p[96];
-                    const float xp[3] = {p0.x, p0.y, p0.z}, vt[3] = {p1.x, p1.y, p1.z};
-                    const float kc[9] = {p2.x, p2.z, p3.x, p2.y, p2.w, p3.y, p3.z, p3.w, *pay_az2(pay, s)};
-                    adj_scatter_global(xp, vt, kc, p0.w, (float)prm.inv_dx, (float)prm.dx, ng, sh.scale[0], sh.scale[2], acc);
-                }
-            }
-        }
         if (wid < kSweepQ)
             sweep_warp<QuadSums<true>, kSweepQ>(sh, sh.qring[wid], (const char *)pay, wid, wid, lane, x0, x1);
         else
@@ -380,6 +312,28 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_adj_sweep(const __grid_con
         if (tid == kSweepThreads - 1) sh.next = sweep_item(take, items);
         __syncthreads();
         now = sh.next;
+    }
+    const unsigned layers = min(head->n_clamped, n_units) * kUnitX;
+    for (unsigned j = blockIdx.x; j < layers; j += gridDim.x) {
+        const int i = clamped[j / kUnitX], u = work[i], layer = (int)(j % kUnitX);
+        int org[3];
+        unit_origin(u, (unsigned)u / kBlockUnits, nb, org);
+        bool any = false;
+        if (tid < 32) {
+            const int g[3] = {org[0] + layer, org[1] + (tid >> 3), org[2] + (tid & 7)};
+            int2 cell = make_int2(0, 0);
+            if (clamped_cell(g, ng)) cell = cells[(long long)i * kUnitCells + 32 * layer + tid];
+            any = cell.y > 0;
+            sh.cell[tid] = cell;
+        } else if (tid == 32) {
+            sh.ng = ng;
+            sh.dx = (float)prm.dx;
+            sh.inv_dx = (float)prm.inv_dx;
+            sh.g0_quad = acc;
+            sh.g0_cubic = acc + 3;
+        }
+        if (__syncthreads_or(any)) scatter_clamped<true, NoMark>(sh, nullptr, (const char *)pay);
+        __syncthreads();
     }
 }
 
@@ -1394,6 +1348,7 @@ __global__ void k_tape_head(const Ctrl *ctrl, TapeHead *head, long long n) {
         head->step = ctrl->step;
         head->time = ctrl->time;
         head->n_work = (unsigned)min((long long)ctrl->n_work, n);
+        head->n_clamped = (unsigned)min((long long)ctrl->n_clamped, n);
     }
     if (threadIdx.x < PM_MAX_COLLIDERS) {
 #pragma unroll
@@ -1426,7 +1381,7 @@ TapeLayout make_tape_layout(long long n, int ng, int slots, int flags) {
     const int nbs = (ng + kBlockEdge - 1) / kBlockEdge;
     const long long nb = (long long)nbs * nbs * nbs;
     const long long nb8 = sort_blocks_per_axis(ng);
-    const long long units = std::max<long long>(1, std::min(n, nb8 * nb8 * nb8 * kBlockUnits));   // listed at most
+    const long long units = listed_units(n, nb8 * nb8 * nb8);
     const long long np = (n + 63) / 64 * 64 > 0 ? (n + 63) / 64 * 64 : 64;
     size_t o = 0;
     T.head = o;    o = align_up(o + sizeof(TapeHead) * (size_t)(slots > 0 ? slots : 1), A);
@@ -1444,6 +1399,7 @@ TapeLayout make_tape_layout(long long n, int ng, int slots, int flags) {
     T.blocks = s;  s = align_up(s + 4 * (size_t)nb, A);
     T.iperm = s;   s = align_up(s + 4 * (size_t)np, A);
     T.work = s;    s = align_up(s + 4 * (size_t)np, A);
+    T.clamped = s; s = align_up(s + 4 * (size_t)units, A);
     T.split = s;   s = align_up(s + (size_t)kUnitCells * (size_t)units, A);
     T.cells = s;   s = align_up(s + 8 * (size_t)kUnitCells * (size_t)units, A);
     T.aff = s;     s = align_up(s + 36 * (size_t)np, A);
@@ -1466,6 +1422,7 @@ void record_redirect(const TapeLayout &T, void *tape, int slot, WS &w) {
     w.block_list = (int *)(b + T.blocks);
     w.slot = (int *)(b + T.iperm);       // the particles' places, the unit list and its cells stay on the tape
     w.work = (int *)(b + T.work);
+    w.clamped = (int *)(b + T.clamped);
     w.rec_cells = (int2 *)(b + T.cells);
     w.rec_split = (unsigned char *)(b + T.split);
     w.tape_aff = (float *)(b + T.aff);
@@ -1508,8 +1465,8 @@ void launch_adjoint(const pm_params &prm, const Parts &pre, const Parts &post, c
             if (dev >= 0 && dev < 64) slots_dev[dev] = slots;
         }
         k_adj_sweep<<<(unsigned)std::min<long long>(slots, n), kSweepThreads, sizeof(SweepShared), s>>>(
-            prm, (const int *)(b + T.work), (const int2 *)(b + T.cells), (const unsigned char *)(b + T.split), h,
-            apay, actl, acc, n);
+            prm, (const int *)(b + T.work), (const int *)(b + T.clamped), (const int2 *)(b + T.cells),
+            (const unsigned char *)(b + T.split), h, apay, actl, acc, n);
     }
     const long long max_items = T.n_blocks * 64;
     const int gb = (int)std::max<long long>(1, std::min<long long>((max_items + 255) / 256, 148LL * 8));

@@ -192,7 +192,7 @@ int pm_p2g(const pm_params *prm, const pm_particles *P, void *ws, size_t ws_byte
     cudaStream_t s = (cudaStream_t)stream;
     // Counters left over from a P2G without a clock since would list blocks twice and move the payload's runs.
     cudaMemsetAsync(&w.ctrl->n_active, 0, sizeof(unsigned), s);
-    cudaMemsetAsync(&w.ctrl->n_work, 0, 4 * sizeof(unsigned), s);
+    cudaMemsetAsync(&w.ctrl->n_work, 0, 5 * sizeof(unsigned), s);
     pm::launch_p2g(pm::PlainScenes{*prm}, pm::make_parts(P), w, s, -1, prm->p2g_ctas_per_sm, prm->stress_ctas_per_sm);
     // The touched blocks are on the list.  The grid update unmarks them too, but it need not follow, and a mark that
     // stays keeps its block off every later list.

@@ -53,7 +53,8 @@ constexpr int kG2PThreads = 256;     // G2P particles per CTA
 // spread over the slots, so the atomics do not queue on one address; cleared by
 // the clock kernel) and the P2G kernel folds the slots into the bounds.  n_work
 // / work_next: the P2G work list of non-empty units and its dynamic cursor;
-// run_next, run_end: the places taken from the two ends of the payload (control
+// run_next, run_end: the places taken from the two ends of the payload;
+// n_clamped: the listed units that hold particles beside the grid's edge (control
 // block 0 of a batch serves all scenes).
 constexpr int kBoundSlots = 128;
 struct Ctrl {
@@ -64,7 +65,7 @@ struct Ctrl {
     unsigned nonfinite;
     unsigned dense_subblocks;   // sub-blocks beyond the fixed-point headroom (status error)
     unsigned mom_bound, mass_bound, dmg_bound;
-    unsigned n_work, work_next, run_next, run_end;   // (cleared together)
+    unsigned n_work, work_next, run_next, run_end, n_clamped;   // (cleared together)
     float col_origin[PM_MAX_COLLIDERS][3];
     float col_vel[PM_MAX_COLLIDERS][3];
     unsigned bound_slots[3][kBoundSlots];   // cleared by the clock kernel
@@ -88,9 +89,15 @@ __host__ __device__ inline int blocked_key_bits(int ng) {
     return b + kSortBlockBits;
 }
 
+// Non-empty units of n particles on n_sblocks sort blocks, at most.
+__host__ __device__ inline long long listed_units(long long n, long long n_sblocks) {
+    const long long all = n_sblocks * kBlockUnits, most = n < all ? n : all;
+    return most > 0 ? most : 1;
+}
+
 struct Layout {
     size_t ctrl, keys_a, keys_b, vals_a, vals_b, hist, block_mask, block_list;
-    size_t g_mom, g_dmg, g_vel, g_gd, payload, inv_perm, work, slot, cells, utot, split, tables, total;
+    size_t g_mom, g_dmg, g_vel, g_gd, payload, inv_perm, work, slot, cells, utot, split, clamped, tables, total;
     int passes, key_bits, n_tiles, nbs;
     long long n_blocks, n_nodes, pay_places;
 };
@@ -132,6 +139,7 @@ __host__ __device__ inline Layout make_layout_sized(long long n, long long n_nod
     L.cells = o;      o = align_up(o + 8 * (size_t)kSortCells * (size_t)n_sblocks, A);   // per cell: first place, count
     L.split = o;      o = align_up(o + (size_t)kSortCells * (size_t)n_sblocks, A);       // per cell, 1 byte
     L.utot = o;       o = align_up(o + 4 * (size_t)kBlockUnits * (size_t)n_sblocks, A);  // per unit: particles
+    L.clamped = o;    o = align_up(o + 4 * (size_t)listed_units(n, n_sblocks), A);
     L.tables = o;     o = align_up(o + table_bytes, A);
     L.total = o;
     return L;
@@ -173,6 +181,7 @@ struct WS {
     const int *perm;
     int *inv_perm;      // particle -> sorted position, written by the last radix pass of pm_bin
     int *work;          // the non-empty units
+    int *clamped;       // places in `work` of the units with cells that need clamped nodes
     int *slot;          // per particle: arrival number in its cell, then payload place
     int2 *cells;        // per cell (unit_key): {first payload place (and kCellRows), particle count}; zero
                         // between substeps
@@ -223,6 +232,7 @@ inline WS make_ws(void *base, const Layout &L) {
     w.cells = (int2 *)(b + L.cells);
     w.utot = (int *)(b + L.utot);
     w.split = (unsigned char *)(b + L.split);
+    w.clamped = (int *)(b + L.clamped);
     w.rec_cells = nullptr;
     w.rec_split = nullptr;
     return w;
@@ -772,12 +782,6 @@ __device__ __forceinline__ void cw5_2(float fx, float e[5]) {
     e[2] = s1 ? w1 : w2;
     e[3] = s1 ? w2 : w3;
     e[4] = s1 ? w3 : 0.0f;
-}
-
-// Adds a value to a fixed-point sum in global memory: one 64-bit atomic.
-__device__ __forceinline__ void red_fix(long long *addr, float v, float scale) {
-    const long long q = to_fix(v, scale);
-    if (q != 0) atomicAdd((unsigned long long *)addr, (unsigned long long)q);
 }
 
 // Brings the line to L2 while the caller does something else.

@@ -17,6 +17,7 @@ __device__ __forceinline__ void reset_ctrl(Ctrl *c, bool shared_counters) {
         c->work_next = 0;
         c->run_next = 0;
         c->run_end = 0;
+        c->n_clamped = 0;
     }
 }
 __device__ __forceinline__ void clear_bound_slots(Ctrl *c, int t) {   // t: 0 .. kBoundSlots - 1

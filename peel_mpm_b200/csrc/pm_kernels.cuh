@@ -35,7 +35,7 @@ void launch_sym_eig(const float *A, long long n, int sweeps, float *ev, float *V
 // particles' APIC affine term and their polar decomposition (R, V, S) and damage
 // drive phi.
 struct TapeLayout {
-    size_t head, actl, acc, adj_q, adj_c, apay, slot0, vel, gd, sw, vpre, blocks, iperm, work, cells, split, aff, pol,
+    size_t head, actl, acc, adj_q, adj_c, apay, slot0, vel, gd, sw, vpre, blocks, iperm, work, clamped, cells, split, aff, pol,
         slot_bytes, total;
     long long n_blocks, aff_stride;
     int slots, flags;

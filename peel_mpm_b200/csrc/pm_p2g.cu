@@ -21,9 +21,9 @@
 // nodes are summed in float registers by a sweep along x and added as exact fixed
 // point (pm_sweep.cuh); integer addition is associative, so the grid sums, and
 // with them the whole substep, are the same bits whatever order the atomics run
-// in.  The 4^3 grid blocks touched are marked and listed.  Particles whose stencil
-// needs the reference's edge clamping (base cell outside [1, n_grid-4]) scatter
-// directly to the global grid instead.
+// in.  The 4^3 grid blocks touched are marked and listed.  Cells whose stencils
+// need the reference's edge clamping (base cell outside [1, n_grid-4]) go straight
+// to the global grid instead (scatter_clamped).
 //
 // Reference: anisompm.py:601-724 (constitutive, damage, P2G) and 768-776
 // (cubic damage scatter).
@@ -302,7 +302,8 @@ __global__ void __launch_bounds__(kCountThreads) k_count(const SC sc, const floa
 // layer goes in rows, from the front of the payload, if those take at most
 // kPayPlaces places per particle, else cell after cell, from the back, so that
 // the two never meet.  Also counts the 4^3-cell sub-blocks beyond the fixed-point
-// headroom.  One warp per unit, one lane per cell of a layer.
+// headroom and lists the units with cells that need clamped nodes.  One warp per
+// unit, one lane per cell of a layer.
 template <class SC>
 __global__ void __launch_bounds__(256) k_offsets(const SC sc, const WS w, long long n) {
     __shared__ int s_morton[8][kUnitCells];
@@ -368,11 +369,27 @@ __global__ void __launch_bounds__(256) k_offsets(const SC sc, const WS w, long l
                 if (w.rec_split) w.rec_split[(long long)i * kUnitCells + 32 * x + lane] = b;
             }
         }
+        const int sid = sc.of_sblock((unsigned)u / kBlockUnits);
+        const int ng = sc.params(sid).n_grid;
+        int org[3];
+        unit_origin(u, (unsigned)u / kBlockUnits - sc.sblock_base(sid), sort_blocks_per_axis(ng), org);
+        if (clamped_unit(org, ng)) {
+            bool any = false;
+#pragma unroll
+            for (int x = 0; x < kUnitX; ++x) {
+                const int g[3] = {org[0] + x, org[1] + y, org[2] + z};
+                any |= c[x] > 0 && clamped_cell(g, ng);
+            }
+            if (__any_sync(0xffffffffu, any) && lane == 0) {
+                const unsigned at = atomicAdd(&w.ctrl->n_clamped, 1u);
+                if (at < n_work) w.clamped[at] = (int)i;   // bounded even without a clock reset
+            }
+        }
         const int mine = c[0] + c[1] + c[2] + c[3];
         const int low = __reduce_add_sync(0xffffffffu, (lane & 7) < 4 ? mine : 0);
         const int high = __reduce_add_sync(0xffffffffu, (lane & 7) < 4 ? 0 : mine);
         if (lane == 0 && max(low, high) > kDenseSubblock)
-            atomicAdd(&w.ctrl[sc.of_sblock((unsigned)u / kBlockUnits)].dense_subblocks,
+            atomicAdd(&w.ctrl[sid].dense_subblocks,
                       (low > kDenseSubblock ? 1u : 0u) + (high > kDenseSubblock ? 1u : 0u));
     }
 }
@@ -580,72 +597,21 @@ __device__ __forceinline__ void mark_node_block(const WS &w, long long gb0, int 
         list_block(w, gb, atomicAdd(&w.ctrl->n_active, 1u));
 }
 
-// Scatter one particle straight into the global grid with the reference's
-// clamped node indices (anisompm.py:716-724, 771-776): the path for particles
-// whose stencil leaves the grid.  `sc` holds the fixed-point scales of
-// {momentum, mass, w d, w}.
-__device__ __noinline__ void scatter_particle_global(const float xp[3], const float mv[3], const float aff[9],
-                                                     float m, float d, float inv_dx, float dx, int ng,
-                                                     const float sc[4], long long *g_mom, long long *g_dmg,
-                                                     const WS &w, long long gb0, int nbs) {
-    {
-        Quad q;
-        quad_weights(xp, inv_dx, ng, q);
-        int NX[3], NY[3], NZ[3];
-        float DX[3], DY[3], DZ[3];
-#pragma unroll
-        for (int o = 0; o < 3; ++o) {
-            NX[o] = clampi(q.b[0] + o, 0, ng - 1);
-            NY[o] = clampi(q.b[1] + o, 0, ng - 1);
-            NZ[o] = clampi(q.b[2] + o, 0, ng - 1);
-            DX[o] = ((float)o - q.fx[0]) * dx;
-            DY[o] = ((float)o - q.fx[1]) * dx;
-            DZ[o] = ((float)o - q.fx[2]) * dx;
-        }
-#pragma unroll
-        for (int ox = 0; ox < 3; ++ox)
-#pragma unroll
-            for (int oy = 0; oy < 3; ++oy) {
-                const float wxy = q.w[ox][0] * q.w[oy][1];
-#pragma unroll
-                for (int oz = 0; oz < 3; ++oz) {
-                    const float wk = wxy * q.w[oz][2];
-                    const float a0 = aff[0] * DX[ox] + aff[1] * DY[oy] + aff[2] * DZ[oz];
-                    const float a1 = aff[3] * DX[ox] + aff[4] * DY[oy] + aff[5] * DZ[oz];
-                    const float a2 = aff[6] * DX[ox] + aff[7] * DY[oy] + aff[8] * DZ[oz];
-                    long long *g = g_mom + 4 * (((long long)NX[ox] * ng + NY[oy]) * ng + NZ[oz]);
-                    red_fix(g, wk * (mv[0] + a0), sc[0]);
-                    red_fix(g + 1, wk * (mv[1] + a1), sc[0]);
-                    red_fix(g + 2, wk * (mv[2] + a2), sc[0]);
-                    red_fix(g + 3, wk * m, sc[1]);
-                    mark_node_block(w, gb0, nbs, NX[ox], NY[oy], NZ[oz]);
-                }
-            }
+struct NodeMark {   // of scatter_clamped
+    static __device__ __forceinline__ void node(const SweepShared &sh, const WS *w, int x, int y, int z) {
+        mark_node_block(*w, sh.gblock, ((int)sh.ng + kBlockEdge - 1) / kBlockEdge, x, y, z);
     }
-    {
-        Cubic c;
-        cubic_weights(xp, inv_dx, ng, c);
-        int NX[4], NY[4], NZ[4];
+};
+
+// Folds a scene's bound slots of quantity v (kept for the grid update too).
+__device__ __forceinline__ void fold_bounds(SweepShared &sh, const WS &w, int sid, int v, int lane) {
+    unsigned m = 0;
 #pragma unroll
-        for (int o = 0; o < 4; ++o) {
-            NX[o] = clampi(c.b[0] + o, 0, ng - 1);
-            NY[o] = clampi(c.b[1] + o, 0, ng - 1);
-            NZ[o] = clampi(c.b[2] + o, 0, ng - 1);
-        }
-#pragma unroll
-        for (int ox = 0; ox < 4; ++ox)
-#pragma unroll
-            for (int oy = 0; oy < 4; ++oy) {
-                const float wxy = c.w[ox][0] * c.w[oy][1];
-#pragma unroll
-                for (int oz = 0; oz < 4; ++oz) {
-                    const float wk = wxy * c.w[oz][2];
-                    long long *g = g_dmg + 2 * (((long long)NX[ox] * ng + NY[oy]) * ng + NZ[oz]);
-                    red_fix(g, wk * d, sc[2]);
-                    red_fix(g + 1, wk, sc[3]);
-                    mark_node_block(w, gb0, nbs, NX[ox], NY[oy], NZ[oz]);
-                }
-            }
+    for (int k = 0; k < kBoundSlots / 32; ++k) m = max(m, w.ctrl[sid].bound_slots[v][k * 32 + lane]);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (lane == 0) {
+        sh.scale[v] = fix_scale(m).scale;
+        (v == 0 ? w.ctrl[sid].mom_bound : v == 1 ? w.ctrl[sid].mass_bound : w.ctrl[sid].dmg_bound) = m;
     }
 }
 
@@ -680,19 +646,9 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_p2g_sweep(const __grid_con
         const pm_params &prm = sc.params(sid);
         const int ng = prm.n_grid, nb = sort_blocks_per_axis(ng), nbs = (ng + kBlockEdge - 1) / kBlockEdge;
         const unsigned blk = gblk - sc.sblock_base(sid);
-        const int org[3] = {(int)(blk / ((unsigned)nb * nb)) * kSortBlock + ((u >> 1) & 1) * kUnitX,
-                            (int)(blk / nb % nb) * kSortBlock + (u & 1) * kUnitY,
-                            (int)(blk % nb) * kSortBlock};   // first cell of the unit
-        if (sid != scene && wid >= 4 && wid < 7) {   // fold the scene's bound slots (kept for the grid update too)
-            unsigned m = 0;
-#pragma unroll
-            for (int k = 0; k < kBoundSlots / 32; ++k) m = max(m, w.ctrl[sid].bound_slots[wid - 4][k * 32 + lane]);
-            m = __reduce_max_sync(0xffffffffu, m);
-            if (lane == 0) {
-                sh.scale[wid - 4] = fix_scale(m).scale;
-                (wid == 4 ? w.ctrl[sid].mom_bound : wid == 5 ? w.ctrl[sid].mass_bound : w.ctrl[sid].dmg_bound) = m;
-            }
-        }
+        int org[3];
+        unit_origin(u, blk, nb, org);
+        if (sid != scene && wid >= 4 && wid < 7) fold_bounds(sh, w, sid, wid - 4, lane);
         scene = sid;
         long long *g_mom = w.g_mom + 4 * sc.node_base(sid);
         long long *g_dmg = w.g_dmg + 2 * sc.node_base(sid);
@@ -704,17 +660,12 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_p2g_sweep(const __grid_con
         }
         // the unit's cells; the table goes back to zero for the next substep
         const int2 next = sh.next;
-        bool edge = false;                // particles that need clamped nodes
-        int2 cell = make_int2(0, 0);
         if (wid >= x0 && wid < x1) {
             cp_async_wait<0>();
-            cell = sh.raw[tid];
-            w.cells[(long long)u * kUnitCells + tid] = make_int2(0, 0);
-            const int c[3] = {tid >> 5, (tid >> 3) & 3, tid & 7};
-            bool reg = true;
-#pragma unroll
-            for (int a = 0; a < 3; ++a) reg = reg && org[a] + c[a] >= 1 && org[a] + c[a] <= ng - 4;
-            edge = cell.y > 0 && !reg;
+            const int2 cell = sh.raw[tid];
+            const int c[3] = {tid >> 5, (tid >> 3) & 3, tid & 7}, g[3] = {org[0] + c[0], org[1] + c[1], org[2] + c[2]};
+            const bool reg = !clamped_cell(g, ng);
+            if (reg) w.cells[(long long)u * kUnitCells + tid] = make_int2(0, 0);   // (the others: below)
             const int cnt = reg ? cell.y : 0;
             sh.cell[tid] = make_int2(cell.x, cnt);
             sh.split[tid] = w.split[(long long)u * kUnitCells + tid];
@@ -734,7 +685,7 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_p2g_sweep(const __grid_con
         } else if (tid == kUnitCells && x0 == 0) {
             w.utot[u] = 0;
         }
-        const bool edges = __syncthreads_or(edge);
+        __syncthreads();
         const long long gb0 = sc.gblock_base(sid);
         // the item after the next is taken, the next one's cells are on their way and the blocks are marked, while
         // this one is swept
@@ -753,22 +704,6 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_p2g_sweep(const __grid_con
         if (next.x >= 0 && wid >= (next.y & 255) && wid < next.y >> 8)
             cp_async8(&sh.raw[tid], w.cells + (long long)next.x * kUnitCells + tid);
         cp_async_commit();
-        if (edges) {                      // the cell's particles over the lanes of its warp
-            const unsigned eb = __ballot_sync(0xffffffffu, edge);
-            for (unsigned m = eb; m; m &= m - 1) {
-                const int l = __ffs(m) - 1;
-                const int f = __shfl_sync(0xffffffffu, cell.x, l), cnt = __shfl_sync(0xffffffffu, cell.y, l);
-                for (int k = lane; k < cnt; k += 32) {
-                    const long long s = place_of(f, k);
-                    const float4 *p = (const float4 *)pay_at(w.payload, s);
-                    const float4 p0 = p[0], p1 = p[32], p2 = p[64], p3 = p[96];
-                    const float xp[3] = {p0.x, p0.y, p0.z}, mv[3] = {p1.x, p1.y, p1.z};
-                    const float aff[9] = {p2.x, p2.z, p3.x, p2.y, p2.w, p3.y, p3.z, p3.w, *pay_az2(w.payload, s)};
-                    scatter_particle_global(xp, mv, aff, p1.w, p0.w, (float)prm.inv_dx, (float)prm.dx, ng, sh.scale, g_mom,
-                                            g_dmg, w, gb0, nbs);
-                }
-            }
-        }
         if (wid < kSweepQ)
             sweep_warp<QuadSums<false>, kSweepQ>(sh, sh.qring[wid], (const char *)w.payload, wid, wid, lane, x0, x1);
         else
@@ -786,6 +721,39 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_p2g_sweep(const __grid_con
         }
         __syncthreads();                  // the item's shared state is done with
         now = next;
+    }
+    const unsigned layers = min(ctrl0->n_clamped, n_units) * kUnitX;
+    for (unsigned i = blockIdx.x; i < layers; i += gridDim.x) {
+        const int u = w.work[w.clamped[i / kUnitX]], layer = (int)(i % kUnitX);
+        const unsigned gblk = (unsigned)u / kBlockUnits;
+        const int sid = sc.of_sblock(gblk);
+        const pm_params &prm = sc.params(sid);
+        const int ng = prm.n_grid;
+        int org[3];
+        unit_origin(u, gblk - sc.sblock_base(sid), sort_blocks_per_axis(ng), org);
+        if (sid != scene && wid >= 4 && wid < 7) fold_bounds(sh, w, sid, wid - 4, lane);
+        scene = sid;
+        bool any = false;
+        if (tid < 32) {
+            int2 *at = w.cells + (long long)u * kUnitCells + 32 * layer + tid;
+            const int g[3] = {org[0] + layer, org[1] + (tid >> 3), org[2] + (tid & 7)};
+            int2 cell = make_int2(0, 0);
+            if (clamped_cell(g, ng)) {
+                cell = *at;
+                *at = make_int2(0, 0);
+            }
+            any = cell.y > 0;
+            sh.cell[tid] = cell;
+        } else if (tid == 32) {
+            sh.ng = ng;
+            sh.dx = (float)prm.dx;
+            sh.inv_dx = (float)prm.inv_dx;
+            sh.g0_quad = w.g_mom + 4 * sc.node_base(sid);
+            sh.g0_cubic = w.g_dmg + 2 * sc.node_base(sid);
+            sh.gblock = sc.gblock_base(sid);
+        }
+        if (__syncthreads_or(any)) scatter_clamped<false, NodeMark>(sh, &w, (const char *)w.payload);
+        __syncthreads();
     }
 }
 

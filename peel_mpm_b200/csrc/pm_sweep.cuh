@@ -112,6 +112,8 @@ struct SweepShared {
     float scale[4];                           // fixed-point scales of {momentum, mass, w d, w}
     long long *g_quad, *g_cubic;              // global sums of the first node of the unit's plane 0
     long long ng;
+    long long *g0_quad, *g0_cubic, gblock;    // scatter_clamped's: global sums of node 0, the scene's first grid block
+    float inv_dx;
     int2 next;                                // the next item (see sweep_item)
     unsigned char mark[36];                   // grid blocks s-1 .. s+1, s-1 .. s+1, s-1 .. s+2 of the unit
 };
@@ -505,6 +507,163 @@ __device__ __forceinline__ void sweep_warp(SweepShared &sh, typename SUMS::Slot 
             dirty = false;
         }
         ox = ox == 0 ? N - 1 : ox - 1;
+    }
+}
+
+// ------------------------------------------------------------ clamped nodes
+// Cells whose stencils need the reference's clamped nodes (anisompm.py:716-724,
+// 771-776; base cell outside [1, n_grid - 4], payload part 0 {x, d}) are left out
+// of the sweep and scattered by the same CTAs when they have run out of items, a
+// layer of a unit (its cells in sh.cell) at a time.  One warp takes up to kClampRun
+// particles of a cell, one after another, and every lane keeps the exact sums of
+// its nodes: lane l quadratic node l of 27, cubic nodes l, l + 32, .. of the 125
+// that the cell's particles can reach, which go to the grid when the run ends or
+// the particles' base cell changes (outside the domain cells share their place in
+// the table).  MARK::node is called for every node that the sums go to.  ADJ: see
+// QuadSums; the cubic sums are CubicLapSums'.
+//
+// A thread per particle with its 236 atomics, a cell of the layer after another,
+// made a substep of a body resting on the upper end of the domain (131k particles,
+// 8 per cell) 595 us, this 82; with four layers pressed into the last one (164k)
+// 1,090 us and 130.  (Called from within the sweep's loop it costs the sweep of bodies
+// that touch no edge 5 to 15%, in registers.)
+__device__ __forceinline__ bool clamped_cell(const int c[3], int ng) {
+    bool reg = true;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) reg = reg && c[a] >= 1 && c[a] <= ng - 4;
+    return !reg;
+}
+// Whether a unit with first cell org has such cells.
+__device__ __forceinline__ bool clamped_unit(const int org[3], int ng) {
+    return org[0] == 0 || org[1] == 0 || org[2] == 0 || org[0] + kUnitX > ng - 3 || org[1] + kUnitY > ng - 3 ||
+           org[2] + kUnitZ > ng - 3;
+}
+// First cell of unit u; blk: its sort block within the scene, nb sort blocks per axis.
+__device__ __forceinline__ void unit_origin(int u, unsigned blk, int nb, int org[3]) {
+    org[0] = (int)(blk / ((unsigned)nb * nb)) * kSortBlock + ((u >> 1) & 1) * kUnitX;
+    org[1] = (int)(blk / nb % nb) * kSortBlock + (u & 1) * kUnitY;
+    org[2] = (int)(blk % nb) * kSortBlock;
+}
+constexpr int kClampRun = 32;
+template <bool ADJ, class MARK>
+__device__ __noinline__ void scatter_clamped(SweepShared &sh, const WS *w, const char *payload) {
+    constexpr int NQ = ADJ ? 3 : 4, NC = ADJ ? 1 : 2, GC = ADJ ? 4 : 2, CN = 4;   // CN: cubic nodes of a lane
+    constexpr unsigned all = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, o[3] = {lane / 9, lane / 3 % 3, lane % 3};
+    const int ng = (int)sh.ng;
+    const float inv_dx = sh.inv_dx, dx = sh.dx;
+    QuadSlot &slot = (&sh.qring[0][0])[wid];       // the rings are idle
+    const int2 mine = sh.cell[lane];
+    int run = 0;
+    for (unsigned todo = __ballot_sync(all, mine.y > 0); todo; todo &= todo - 1) {
+        const int l = __ffs(todo) - 1;
+        const int first = __shfl_sync(all, mine.x, l), cnt = __shfl_sync(all, mine.y, l);
+        for (int k0 = 0; k0 < cnt; k0 += kClampRun, ++run) {
+            if ((run & 7) != wid) continue;
+            // lane k: the run's k-th particle, to shared memory; its base cell and place between the nodes
+            const int n = min(cnt - k0, kClampRun);
+            float f[3] = {0.0f, 0.0f, 0.0f};
+            int b[3] = {0, 0, 0};
+            __syncwarp();                          // the run before is done with
+            if (lane < n) {
+                const long long s = place_of(first, k0 + lane);
+                const float4 *p = (const float4 *)(payload + (s >> 5) * kPayBlock + (s & 31) * 16);
+                const float4 p0 = p[0];
+                slot.p[0][lane] = p0;
+#pragma unroll
+                for (int j = 1; j < 4; ++j) slot.p[j][lane] = p[32 * j];
+                slot.az2[lane] = ((const float *)(payload + (s >> 5) * kPayBlock + 2048))[s & 31];
+                const float xp[3] = {p0.x, p0.y, p0.z};
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    const float X = __fmul_rn(xp[a], inv_dx), fb = floorf(__fsub_rn(X, 0.5f));
+                    b[a] = sat_base(fb, ng);
+                    f[a] = __fsub_rn(X, fb);
+                }
+            }
+            __syncwarp();
+            bool other = false;                    // another base cell than the particle before
+#pragma unroll
+            for (int a = 0; a < 3; ++a) other |= __shfl_up_sync(all, b[a], 1) != b[a];
+            const unsigned ends = __ballot_sync(all, lane == 0 || lane >= n || other) >> 1;   // bit k: k is the last of its base
+            long long q[NQ], c[CN][NC];
+#pragma unroll
+            for (int i = 0; i < NQ; ++i) q[i] = 0;
+#pragma unroll
+            for (int j = 0; j < CN; ++j)
+#pragma unroll
+                for (int i = 0; i < NC; ++i) c[j][i] = 0;
+            for (int k = 0; k < n; ++k) {
+                const float4 p1 = slot.p[1][k], p2 = slot.p[2][k], p3 = slot.p[3][k];
+                const float a22 = slot.az2[k], d = slot.p[0][k].w;
+                const float fk[3] = {__shfl_sync(all, f[0], k), __shfl_sync(all, f[1], k), __shfl_sync(all, f[2], k)};
+                // lane 5 a + i: the cubic weight of axis a, node i
+                const float fl = lane < 5 ? fk[0] : (lane < 10 ? fk[1] : fk[2]);
+                const int il = lane < 5 ? lane : (lane < 10 ? lane - 5 : lane - 10);
+                const float wl = cw5_node(il, fl), wl2 = ADJ ? cw5_2_node(il, fl) : 0.0f;
+                {   // quadratic: this lane's node (lanes 27 and up: not used)
+                    float wq[3], D[3];
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        const float t = o[a] == 0 ? 1.5f - fk[a] : (o[a] == 1 ? fk[a] - 1.0f : fk[a] - 0.5f);
+                        wq[a] = o[a] == 1 ? 0.75f - t * t : 0.5f * (t * t);
+                        D[a] = ((float)o[a] - fk[a]) * dx;
+                    }
+                    const float wk = wq[0] * wq[1] * wq[2], sm = sh.scale[0];
+                    const float a0 = p2.x * D[0] + p2.z * D[1] + p3.x * D[2];
+                    const float a1 = p2.y * D[0] + p2.w * D[1] + p3.y * D[2];
+                    const float a2 = p3.z * D[0] + p3.w * D[1] + a22 * D[2];
+                    q[0] = fix_add(q[0], to_fix(wk * (p1.x + a0), sm));
+                    q[1] = fix_add(q[1], to_fix(wk * (p1.y + a1), sm));
+                    q[2] = fix_add(q[2], to_fix(wk * (p1.z + a2), sm));
+                    if (!ADJ) q[NQ - 1] = fix_add(q[NQ - 1], to_fix(wk * p1.w, sh.scale[1]));
+                }
+#pragma unroll
+                for (int j = 0; j < CN; ++j) {     // (lanes past the 125th node: any weight, not used)
+                    const int m = min(lane + 32 * j, 124), nx = m / 25, ny = 5 + m / 5 % 5, nz = 10 + m % 5;
+                    const float wx = __shfl_sync(all, wl, nx), wy = __shfl_sync(all, wl, ny), wz = __shfl_sync(all, wl, nz);
+                    if (ADJ) {
+                        const float vx = __shfl_sync(all, wl2, nx), vy = __shfl_sync(all, wl2, ny),
+                                    vz = __shfl_sync(all, wl2, nz);
+                        const float ab = d * (vx * wy + wx * vy), e = d * (wx * wy);
+                        c[j][0] = fix_add(c[j][0], to_fix(ab * wz + e * vz, sh.scale[2]));
+                    } else {
+                        const float wk = wx * wy * wz;
+                        c[j][0] = fix_add(c[j][0], to_fix(wk * d, sh.scale[2]));
+                        c[j][NC - 1] = fix_add(c[j][NC - 1], to_fix(wk, sh.scale[3]));
+                    }
+                }
+                if (k < n - 1 && !(ends >> k & 1)) continue;
+                const int bk[3] = {__shfl_sync(all, b[0], k), __shfl_sync(all, b[1], k), __shfl_sync(all, b[2], k)};
+                if (lane < 27) {
+                    const int x = clampi(bk[0] + o[0], 0, ng - 1), y = clampi(bk[1] + o[1], 0, ng - 1),
+                              z = clampi(bk[2] + o[2], 0, ng - 1);
+                    long long *g = sh.g0_quad + 4 * (((long long)x * ng + y) * ng + z);
+#pragma unroll
+                    for (int i = 0; i < NQ; ++i) {
+                        if (q[i] != 0) red_add(g + i, q[i]);
+                        q[i] = 0;
+                    }
+                    MARK::node(sh, w, x, y, z);
+                }
+#pragma unroll
+                for (int j = 0; j < CN; ++j) {
+                    const int m = lane + 32 * j;
+                    if (m < 125) {
+                        const int x = clampi(bk[0] - 1 + m / 25, 0, ng - 1), y = clampi(bk[1] - 1 + m / 5 % 5, 0, ng - 1),
+                                  z = clampi(bk[2] - 1 + m % 5, 0, ng - 1);
+                        long long *g = sh.g0_cubic + GC * (((long long)x * ng + y) * ng + z);
+#pragma unroll
+                        for (int i = 0; i < NC; ++i) {
+                            if (c[j][i] != 0) red_add(g + i, c[j][i]);
+                            c[j][i] = 0;
+                        }
+                        MARK::node(sh, w, x, y, z);
+                    }
+                }
+                __syncwarp();
+            }
+        }
     }
 }
 
