@@ -395,11 +395,8 @@ __global__ void __launch_bounds__(256) k_offsets(const SC sc, const WS w, long l
 }
 
 // Particle ids by place, in order of arrival.  Particles of cells of more than
-// kRankRows particles are marked in w.slot (see k_rank); those of more than
-// kRankMost, four times what the fixed-point headroom allows a whole sub-block
-// (dense_subblocks reports them; also where positions that are not numbers
-// gather), stay in order of arrival.
-constexpr int kRankRows = 64, kRankWarps = 4, kRankMost = 4 * kDenseSubblock;
+// kRankRows particles are marked in w.slot (see k_rank).
+constexpr int kRankRows = 64, kRankWarps = 4, kRankRun = kRankRows * 32 / kRankWarps;
 template <class SC>
 __global__ void __launch_bounds__(256) k_place(const SC sc, const float *__restrict__ x, long long n, long long ps,
                                                const WS w) {
@@ -412,7 +409,37 @@ __global__ void __launch_bounds__(256) k_place(const SC sc, const float *__restr
     const int2 cell = w.cells[cell_of(sc, sid, xp, prm.n_grid, (float)prm.inv_dx)];
     const long long at = place_of(cell.x, slot);
     w.ids[at] = (int)p;
-    if (cell.y > kRankRows) w.slot[p] = cell.y > kRankMost ? (int)at : -1;
+    if (cell.y > kRankRows) w.slot[p] = -1;
+}
+
+// Sorts the ids of a layer's cells `more` (cell: this lane's), each in runs of
+// kRankRun, a warp to a run (buf: this warp's).
+__device__ __noinline__ void sort_runs(int *ids, int2 cell, unsigned more, int *buf) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int run = 0; more; more &= more - 1) {
+        const int l = __ffs(more) - 1;
+        const int first = __shfl_sync(0xffffffffu, cell.x, l), total = __shfl_sync(0xffffffffu, cell.y, l);
+        const int base = first & ~kCellRows, step = first < 0 ? 32 : 1;
+        for (int k0 = 0; k0 < total; k0 += kRankRun, ++run) {
+            if (run % kRankWarps != wid) continue;
+            const int n = min(kRankRun, total - k0);
+            for (int k = lane; k < kRankRun; k += 32) buf[k] = k < n ? ids[base + (k0 + k) * step] : 0x7fffffff;
+            __syncwarp();
+            for (int k = 2; k <= kRankRun; k *= 2)           // bitonic
+                for (int j = k / 2; j > 0; j /= 2) {
+                    for (int q = lane; q < kRankRun / 2; q += 32) {
+                        const int a = 2 * q - (q & (j - 1)), va = buf[a], vb = buf[a + j];
+                        if ((va > vb) == ((a & k) == 0)) {
+                            buf[a] = vb;
+                            buf[a + j] = va;
+                        }
+                    }
+                    __syncwarp();
+                }
+            for (int k = lane; k < n; k += 32) ids[base + (k0 + k) * step] = buf[k];
+            __syncwarp();
+        }
+    }
 }
 
 // Gives every particle its payload place (w.slot): in its cell's run by rank of
@@ -424,8 +451,12 @@ __global__ void __launch_bounds__(256) k_place(const SC sc, const float *__restr
 // at 27 per cell, 11 here; sorting the columns by insertion, or skipping
 // columns that arrived in order, was slower: longer chains.)  Cells of more than
 // kRankRows particles are left to k_stress, where every particle counts for
-// itself.  (Counted in k_stress for every cell, reading the ids from global
-// memory: 956 us there against 715 and 85 here, 8.8M particles at 27 per cell.)
+// itself, reading the ids from global memory (for every cell: 956 us there against
+// 715 and 85 here, 8.8M particles at 27 per cell); of more than kRankRun in runs that
+// are sorted here, so that it counts by halving: 2,000 particles without a position,
+// in one cell, 190 us there and 33 now, and no cell need be left in order of
+// arrival.  (Runs from kRankRows on: 512k particles at 125 per cell 255 us per
+// substep against 224, 885k at 216 per cell 359 against 380.)
 __global__ void __launch_bounds__(32 * kRankWarps) k_rank(const WS w, long long n) {
     __shared__ int ids[kRankRows][32];
     const unsigned n_layers = min(w.ctrl->n_work, (unsigned)min(n, (long long)0x1fffffff)) * kUnitX;
@@ -456,6 +487,11 @@ __global__ void __launch_bounds__(32 * kRankWarps) k_rank(const WS w, long long 
 #pragma unroll
             for (int q = 0; q < 4; ++q)
                 if (id[q] >= 0) w.slot[id[q]] = (cell.x & ~kCellRows) + rank[q] * step;
+        }
+        const unsigned more = __ballot_sync(0xffffffffu, cell.y > kRankRun);   // the same in every warp
+        if (more) {
+            __syncthreads();                 // the columns are ranked
+            sort_runs(w.ids, cell, more, &ids[0][0] + wid * kRankRun);
         }
     }
 }
@@ -529,7 +565,18 @@ __global__ void __launch_bounds__(256, MINB) k_stress(const SC sc, const Parts P
         const int *ids = w.ids + (cell.x & ~kCellRows);
         const long long step = cell.x < 0 ? 32 : 1;
         int rank = 0;
-        for (int k = 0; k < cell.y; ++k) rank += ids[k * step] < (int)p;
+        if (cell.y <= kRankRun) {
+            for (int k = 0; k < cell.y; ++k) rank += ids[k * step] < (int)p;
+        } else {                                                     // sorted runs: how many ids of each are smaller
+            for (int k0 = 0; k0 < cell.y; k0 += kRankRun) {
+                int lo = k0, hi = min(k0 + kRankRun, cell.y);
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (ids[mid * step] < (int)p) lo = mid + 1; else hi = mid;
+                }
+                rank += lo - k0;
+            }
+        }
         s = place_of(cell.x, rank);
         w.slot[p] = (int)s;                                          // (a recorded substep keeps it)
     }
