@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(kCountThreads) k_count(const SC sc, const floa
 // unit, one lane per cell of a layer.
 template <class SC>
 __global__ void __launch_bounds__(256) k_offsets(const SC sc, const WS w, long long n) {
-    __shared__ int s_morton[8][kUnitCells];
+    __shared__ __align__(16) int s_morton[8][kUnitCells];   // read as int4 too
     const unsigned n_work = min(w.ctrl->n_work, (unsigned)min(n, (long long)0x7fffffff));
     const int lane = threadIdx.x & 31;
     int *morton = s_morton[threadIdx.x >> 5];
