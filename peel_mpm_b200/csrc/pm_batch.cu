@@ -70,7 +70,7 @@ int make_plan(int32_t S, const int64_t *n, const int32_t *ng, BatchPlan &bp) {
     bp.n_gblocks = bp.gblk[S];
     bp.n_sblocks = bp.sblk[S];
     bp.n_ctas = bp.ctab[S];
-    if (bp.n_total >= (1LL << 31)) return report_error(PM_ERR_ARG, "batch particle count must be < 2^31");
+    if (bp.n_total > pm::kMaxParticles) return report_error(PM_ERR_ARG, "batch particle count must be at most 2^30 - 32");
     if (bp.n_gblocks >= (1LL << 31)) return report_error(PM_ERR_ARG, "batch grid is too large");
     const int key_bits = bits_for((unsigned long long)bp.n_sblocks) + pm::kSortBlockBits;
     if (key_bits > 32) return report_error(PM_ERR_ARG, "batch has more than 2^23 sort blocks");

@@ -57,7 +57,7 @@ int check_params(const pm_params *prm) {
 
 int check_particles(const pm_particles *P, bool need_all) {
     if (!P) return fail(PM_ERR_ARG, "particles is NULL");
-    if (P->n < 0 || P->n >= (1LL << 31)) return fail(PM_ERR_ARG, "particle count must be in [0, 2^31)");
+    if (P->n < 0 || P->n > pm::kMaxParticles) return fail(PM_ERR_ARG, "particle count must be in [0, 2^30 - 32]");
     if (P->plane_stride < P->n) return fail(PM_ERR_ARG, "plane_stride < n");
     if (!P->x) return fail(PM_ERR_ARG, "x is NULL");
     if (need_all) {
@@ -72,6 +72,7 @@ int check_particles(const pm_particles *P, bool need_all) {
 int get_ws(void *ws, size_t bytes, long long n, int ng, pm::WS *out) {
     if (!ws) return fail(PM_ERR_WORKSPACE, "workspace is NULL");
     if (((uintptr_t)ws & 255) != 0) return fail(PM_ERR_WORKSPACE, "workspace must be 256-byte aligned");
+    if (n > pm::kMaxParticles) return fail(PM_ERR_ARG, "particle count must be at most 2^30 - 32");
     const pm::Layout L = pm::make_layout(n, ng);
     if (bytes < L.total) return fail(PM_ERR_WORKSPACE, "workspace too small for (n, n_grid)");
     *out = pm::make_ws(ws, L);
@@ -124,14 +125,14 @@ int pm_prepare(void) {
 
 int pm_workspace_size(int64_t n, int32_t n_grid, size_t *bytes) {
     if (!bytes) return fail(PM_ERR_ARG, "bytes is NULL");
-    if (n < 0 || n_grid < 4 || n_grid > 1024) return fail(PM_ERR_ARG, "bad n or n_grid");
+    if (n < 0 || n > pm::kMaxParticles || n_grid < 4 || n_grid > 1024) return fail(PM_ERR_ARG, "bad n or n_grid");
     *bytes = pm::make_layout(n, n_grid).total;
     return PM_OK;
 }
 
 int pm_workspace_layout(int64_t n, int32_t n_grid, pm_ws_layout *out) {
     if (!out) return fail(PM_ERR_ARG, "out is NULL");
-    if (n < 0 || n_grid < 4 || n_grid > 1024) return fail(PM_ERR_ARG, "bad n or n_grid");
+    if (n < 0 || n > pm::kMaxParticles || n_grid < 4 || n_grid > 1024) return fail(PM_ERR_ARG, "bad n or n_grid");
     const pm::Layout L = pm::make_layout(n, n_grid);
     out->ctrl = L.ctrl; out->keys_a = L.keys_a; out->keys_b = L.keys_b; out->vals_a = L.vals_a;
     out->vals_b = L.vals_b; out->hist = L.hist; out->block_mask = L.block_mask; out->block_list = L.block_list;
@@ -266,7 +267,8 @@ static int tape_flags(const pm_params *prm) { return prm->n_colliders > 0 ? PM_T
 
 int pm_tape_size(int64_t n, int32_t n_grid, int32_t slots, int32_t flags, size_t *bytes) {
     if (!bytes) return fail(PM_ERR_ARG, "bytes is NULL");
-    if (n < 0 || n_grid < 4 || n_grid > 1024 || slots < 1) return fail(PM_ERR_ARG, "bad n, n_grid or slots");
+    if (n < 0 || n > pm::kMaxParticles || n_grid < 4 || n_grid > 1024 || slots < 1)
+        return fail(PM_ERR_ARG, "bad n, n_grid or slots");
     if (flags & ~PM_TAPE_COLLIDERS) return fail(PM_ERR_ARG, "unknown tape flags");
     *bytes = pm::make_tape_layout(n, n_grid, slots, flags).total;
     return PM_OK;
@@ -276,7 +278,7 @@ int pm_tape_init(void *tape, size_t tape_bytes, int64_t n, int32_t n_grid, int32
                  void *stream) {
     int rc;
     if ((rc = check_device())) return rc;
-    if (n < 0 || n_grid < 4 || n_grid > 1024) return fail(PM_ERR_ARG, "bad n or n_grid");
+    if (n < 0 || n > pm::kMaxParticles || n_grid < 4 || n_grid > 1024) return fail(PM_ERR_ARG, "bad n or n_grid");
     if (flags & ~PM_TAPE_COLLIDERS) return fail(PM_ERR_ARG, "unknown tape flags");
     pm::TapeLayout T;
     if ((rc = get_tape(tape, tape_bytes, n, n_grid, slots, flags, 0, &T))) return rc;

@@ -25,6 +25,8 @@ constexpr int kBlockUnits = kSortCells / kUnitCells;
 constexpr int kPayPlaces = 2;
 constexpr int kPayBytes = 68;         // of a place: 4 float4 and 1 float
 constexpr int kCellRows = 1 << 31;    // in a cell's first place: its layer is in rows
+// Places are numbered in the 31 bits below kCellRows.
+constexpr long long kMaxParticles = (1LL << 31) / kPayPlaces - 32;
 constexpr int kSortThreads = 256;
 constexpr int kSortItems = 16;
 constexpr int kSortTile = kSortThreads * kSortItems;   // keys per radix tile
