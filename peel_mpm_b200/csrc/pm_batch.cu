@@ -83,7 +83,7 @@ int make_plan(int32_t S, const int64_t *n, const int32_t *ng, BatchPlan &bp) {
     bp.off_sblk = o;  o = pm::align_up(o + arr, A);
     bp.off_gblk = o;  o = pm::align_up(o + arr, A);
     bp.off_ctab = o;  o = pm::align_up(o + arr, A);
-    bp.L = pm::make_layout_sized(bp.n_total, bp.n_nodes, bp.n_gblocks, bp.n_sblocks, key_bits, S, o);
+    bp.L = pm::make_layout_sized(bp.n_total, bp.n_nodes, bp.n_gblocks, bp.n_sblocks, 0, key_bits, S, o);
     bp.off_prms += bp.L.tables;
     bp.off_pb += bp.L.tables;
     bp.off_nodeb += bp.L.tables;

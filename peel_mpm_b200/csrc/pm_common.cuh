@@ -105,28 +105,29 @@ struct Layout {
 };
 
 // n particles, n_nodes grid nodes, n_blocks 4^3 grid blocks, n_sblocks 8^3-cell
-// sort blocks, sort keys of key_bits bits, n_ctrl control blocks and table_bytes
-// of scene tables.
+// sort blocks, sort keys of key_bits bits for n_sort particles (pm_bin's and
+// pm_bin_sort's; 0 for a batch, which sorts nothing), n_ctrl control blocks and
+// table_bytes of scene tables.
 __host__ __device__ inline Layout make_layout_sized(long long n, long long n_nodes, long long n_blocks,
-                                                    long long n_sblocks, int key_bits, int n_ctrl,
+                                                    long long n_sblocks, long long n_sort, int key_bits, int n_ctrl,
                                                     size_t table_bytes) {
     Layout L;
     const size_t A = 256;
-    L.n_tiles = (int)((n + kSortTile - 1) / kSortTile);
+    L.n_tiles = (int)((n_sort + kSortTile - 1) / kSortTile);
     if (L.n_tiles < 1) L.n_tiles = 1;
     L.key_bits = key_bits < 1 ? 1 : key_bits;
     L.passes = radix_passes(L.key_bits);
     L.nbs = 0;
     L.n_blocks = n_blocks;
     L.n_nodes = n_nodes;
-    size_t nn = (size_t)(n > 0 ? n : 1);
+    const size_t nn = (size_t)(n > 0 ? n : 1), ns = (size_t)(n_sort > 0 ? n_sort : 1);
     L.pay_places = (kPayPlaces * (long long)nn + 31) / 32 * 32;
     size_t o = 0;
     L.ctrl = o;       o = align_up(o + sizeof(Ctrl) * (size_t)(n_ctrl > 0 ? n_ctrl : 1), A);
-    L.keys_a = o;     o = align_up(o + 4 * nn, A);
-    L.keys_b = o;     o = align_up(o + 4 * nn, A);
-    L.vals_a = o;     o = align_up(o + 4 * nn, A);
-    L.vals_b = o;     o = align_up(o + 4 * nn, A);
+    L.keys_a = o;     o = align_up(o + 4 * ns, A);
+    L.keys_b = o;     o = align_up(o + 4 * ns, A);
+    L.vals_a = o;     o = align_up(o + 4 * ns, A);
+    L.vals_b = o;     o = align_up(o + 4 * ns, A);
     L.hist = o;       o = align_up(o + 4 * ((size_t)kRadixTop * L.n_tiles + kRadixTop), A);
     L.block_mask = o; o = align_up(o + (size_t)L.n_blocks, A);
     L.block_list = o; o = align_up(o + 4 * (size_t)L.n_blocks, A);
@@ -134,13 +135,13 @@ __host__ __device__ inline Layout make_layout_sized(long long n, long long n_nod
     L.g_dmg = o;      o = align_up(o + 16 * (size_t)L.n_nodes, A);   // 2 x int64 fixed point per node
     L.g_vel = o;      o = align_up(o + 16 * (size_t)L.n_nodes, A);
     L.g_gd = o;       o = align_up(o + 4 * (size_t)L.n_nodes, A);
-    L.payload = o;    o = align_up(o + 80 * (size_t)L.pay_places, A);     // 5 float4 parts per place
-    L.inv_perm = o;   o = align_up(o + 4 * nn, A);
+    L.payload = o;    o = align_up(o + (kPayBytes + 4) * (size_t)L.pay_places, A);   // the payload, then the ids
+    L.inv_perm = o;   o = align_up(o + 4 * ns, A);
     L.work = o;       o = align_up(o + 4 * nn, A);                    // the non-empty units
     L.slot = o;       o = align_up(o + 4 * nn, A);                    // a particle's payload place
     L.cells = o;      o = align_up(o + 8 * (size_t)kSortCells * (size_t)n_sblocks, A);   // per cell: first place, count
     L.split = o;      o = align_up(o + (size_t)kSortCells * (size_t)n_sblocks, A);       // per cell, 1 byte
-    L.utot = o;       o = align_up(o + 4 * (size_t)kBlockUnits * (size_t)n_sblocks, A);  // per unit: particles
+    L.utot = o;       o = align_up(o + 4 * (size_t)kBlockUnits * (size_t)n_sblocks, A);  // per unit: cells reached
     L.clamped = o;    o = align_up(o + 4 * (size_t)listed_units(n, n_sblocks), A);
     L.tables = o;     o = align_up(o + table_bytes, A);
     L.total = o;
@@ -153,7 +154,7 @@ __host__ __device__ inline Layout make_layout(long long n, int ng) {
     const int nbs = (ng + kBlockEdge - 1) / kBlockEdge;
     const int kb = sort_bits(ng) > blocked_key_bits(ng) ? sort_bits(ng) : blocked_key_bits(ng);
     const long long nb8 = sort_blocks_per_axis(ng);
-    Layout L = make_layout_sized(n, (long long)ng * ng * ng, (long long)nbs * nbs * nbs, nb8 * nb8 * nb8, kb, 1, 0);
+    Layout L = make_layout_sized(n, (long long)ng * ng * ng, (long long)nbs * nbs * nbs, nb8 * nb8 * nb8, n, kb, 1, 0);
     L.nbs = nbs;
     return L;
 }
