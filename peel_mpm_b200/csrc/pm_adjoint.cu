@@ -268,6 +268,7 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_adj_sweep(const __grid_con
     const int ng = prm.n_grid, nb = sort_blocks_per_axis(ng);
     for (int i = tid; i < kSweepQ * 4 * kQRows * kPlaneCols; i += kSweepThreads) sh.qpl[0][0][i] = 0;
     for (int i = tid; i < kSweepC * 2 * kCRows * kPlaneCols; i += kSweepThreads) sh.cpl[0][0][i] = 0;
+    if (tid == 0) sh.clamped_layers = min(head->n_clamped, n_units) * kUnitX;
     if (wid >= 4 && wid < 6) {            // fold the bound slots (kept for the grid adjoint too)
         unsigned m = 0;
 #pragma unroll
@@ -313,8 +314,7 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_adj_sweep(const __grid_con
         __syncthreads();
         now = sh.next;
     }
-    const unsigned layers = min(head->n_clamped, n_units) * kUnitX;
-    for (unsigned j = blockIdx.x; j < layers; j += gridDim.x) {
+    for (unsigned j = blockIdx.x; j < sh.clamped_layers; j += gridDim.x) {
         const int i = clamped[j / kUnitX], u = work[i], layer = (int)(j % kUnitX);
         int org[3];
         unit_origin(u, (unsigned)u / kBlockUnits, nb, org);

@@ -678,6 +678,7 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_p2g_sweep(const __grid_con
     if (tid < 36) sh.mark[tid] = 0;
     if (tid == 0) {
         sh.scale[3] = fix_scale(__float_as_uint(1.0f)).scale;
+        sh.clamped_layers = min(ctrl0->n_clamped, n_units) * kUnitX;
         sh.next = sweep_unit(gridDim.x + atomicAdd(&ctrl0->work_next, 1u), items, w.work);
     }
     int2 now = sweep_unit(blockIdx.x, items, w.work);    // the first item is the CTA's own
@@ -769,8 +770,7 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_p2g_sweep(const __grid_con
         __syncthreads();                  // the item's shared state is done with
         now = next;
     }
-    const unsigned layers = min(ctrl0->n_clamped, n_units) * kUnitX;
-    for (unsigned i = blockIdx.x; i < layers; i += gridDim.x) {
+    for (unsigned i = blockIdx.x; i < sh.clamped_layers; i += gridDim.x) {
         const int u = w.work[w.clamped[i / kUnitX]], layer = (int)(i % kUnitX);
         const unsigned gblk = (unsigned)u / kBlockUnits;
         const int sid = sc.of_sblock(gblk);

@@ -114,6 +114,7 @@ struct SweepShared {
     long long ng;
     long long *g0_quad, *g0_cubic, gblock;    // scatter_clamped's: global sums of node 0, the scene's first grid block
     float inv_dx;
+    unsigned clamped_layers;                  // layers of the units that scatter_clamped takes
     int2 next;                                // the next item (see sweep_item)
     unsigned char mark[36];                   // grid blocks s-1 .. s+1, s-1 .. s+1, s-1 .. s+2 of the unit
 };
