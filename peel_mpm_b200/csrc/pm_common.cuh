@@ -296,8 +296,6 @@ __device__ __forceinline__ int upper_index(const long long *a, int n, long long 
 struct PlainScenes {
     pm_params prm;
     static constexpr bool batched = false;
-    int count() const { return 1; }
-    __device__ __forceinline__ int of_particle(long long) const { return 0; }
     __device__ __forceinline__ int of_sblock(unsigned) const { return 0; }
     __device__ __forceinline__ int of_gblock(long long) const { return 0; }
     __device__ __forceinline__ int of_cta(long long) const { return 0; }
@@ -319,8 +317,6 @@ struct BatchScenes {
     const long long *ctab;        // first G2P CTA, [n + 1]
     int n;
     static constexpr bool batched = true;
-    int count() const { return n; }
-    __device__ __forceinline__ int of_particle(long long p) const { return upper_index(pb, n, p); }
     __device__ __forceinline__ int of_sblock(unsigned b) const { return upper_index(sblk, n, (long long)b); }
     __device__ __forceinline__ int of_gblock(long long b) const { return upper_index(gblk, n, b); }
     __device__ __forceinline__ int of_cta(long long c) const { return upper_index(ctab, n, c); }

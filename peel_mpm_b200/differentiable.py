@@ -194,7 +194,7 @@ def auto_segment(sim: AnisoMPM, n_steps: int, memory_fraction: float = 0.5) -> i
     """The longest segment (at most ``n_steps``) whose recording fits in
     ``memory_fraction`` of the device's free memory.  A segment as long as
     the rollout records every substep during the forward, so the backward
-    recomputes nothing (1M particles on 128^3: ~0.23 GB per substep)."""
+    recomputes nothing (1M particles on 128^3: ~0.32 GB per substep)."""
     free, _ = torch.cuda.mem_get_info(sim.device)
     budget = int(free * memory_fraction)
     lo, hi = 1, max(1, int(n_steps))
