@@ -461,6 +461,7 @@ __global__ void __launch_bounds__(32 * kRankWarps) k_rank(const WS w, long long 
     __shared__ int ids[kRankRows][32];
     const unsigned n_layers = min(w.ctrl->n_work, (unsigned)min(n, (long long)0x1fffffff)) * kUnitX;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    bool crowded = false;
     for (unsigned i = blockIdx.x; i < n_layers; i += gridDim.x) {
         const int2 cell = w.cells[(long long)w.work[i / kUnitX] * kUnitCells + 32 * (i % kUnitX) + lane];
         const int cnt = cell.y <= kRankRows ? cell.y : 0;
@@ -488,11 +489,13 @@ __global__ void __launch_bounds__(32 * kRankWarps) k_rank(const WS w, long long 
             for (int q = 0; q < 4; ++q)
                 if (id[q] >= 0) w.slot[id[q]] = (cell.x & ~kCellRows) + rank[q] * step;
         }
+        crowded |= cell.y > kRankRun;
+    }
+    if (!__syncthreads_or(crowded)) return;  // the columns are ranked
+    for (unsigned i = blockIdx.x; i < n_layers; i += gridDim.x) {
+        const int2 cell = w.cells[(long long)w.work[i / kUnitX] * kUnitCells + 32 * (i % kUnitX) + lane];
         const unsigned more = __ballot_sync(0xffffffffu, cell.y > kRankRun);   // the same in every warp
-        if (more) {
-            __syncthreads();                 // the columns are ranked
-            sort_runs(w.ids, cell, more, &ids[0][0] + wid * kRankRun);
-        }
+        if (more) sort_runs(w.ids, cell, more, &ids[0][0] + wid * kRankRun);
     }
 }
 
