@@ -265,6 +265,7 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_adj_sweep(const __grid_con
     const int lane = tid & 31, wid = __reduce_max_sync(0xffffffffu, tid >> 5);
     const unsigned n_units = min(head->n_work, (unsigned)min(n, (long long)0x1fffffff));
     const SweepItems items = sweep_items(n_units);
+    const bool cloud = n < (long long)kCloud * n_units;
     const int ng = prm.n_grid, nb = sort_blocks_per_axis(ng);
     for (int i = tid; i < kSweepQ * 4 * kQRows * kPlaneCols; i += kSweepThreads) sh.qpl[0][0][i] = 0;
     for (int i = tid; i < kSweepC * 2 * kCRows * kPlaneCols; i += kSweepThreads) sh.cpl[0][0][i] = 0;
@@ -293,8 +294,8 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_adj_sweep(const __grid_con
             const int cnt = clamped_cell(g, ng) ? 0 : cell.y;
             sh.cell[tid] = make_int2(cell.x, cnt);
             sh.split[tid] = split[(long long)i * kUnitCells + tid];
-            const int rows = __reduce_max_sync(0xffffffffu, cnt);
-            if (lane == 0) sh.layer_rows[wid] = rows;
+            const int code = layer_code(cnt, cloud);
+            if (lane == 0) sh.layer_rows[wid] = code;
         }
         if (tid == kSweepThreads - 1) {
             sh.ng = ng;

@@ -676,6 +676,7 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_p2g_sweep(const __grid_con
     Ctrl *ctrl0 = w.ctrl;
     const unsigned n_units = min(ctrl0->n_work, (unsigned)min(n, (long long)0x1fffffff));
     const SweepItems items = sweep_items(n_units);
+    const bool cloud = n < (long long)kCloud * n_units;
     for (int i = tid; i < kSweepQ * 4 * kQRows * kPlaneCols; i += kSweepThreads) sh.qpl[0][0][i] = 0;
     for (int i = tid; i < kSweepC * 2 * kCRows * kPlaneCols; i += kSweepThreads) sh.cpl[0][0][i] = 0;
     if (tid < 36) sh.mark[tid] = 0;
@@ -720,8 +721,8 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_p2g_sweep(const __grid_con
             const int cnt = reg ? cell.y : 0;
             sh.cell[tid] = make_int2(cell.x, cnt);
             sh.split[tid] = w.split[(long long)u * kUnitCells + tid];
-            const int rows = __reduce_max_sync(0xffffffffu, cnt);
-            if (lane == 0) sh.layer_rows[wid] = rows;
+            const int code = layer_code(cnt, cloud);
+            if (lane == 0) sh.layer_rows[wid] = code;
             if (cnt > 0) {
                 // the cell's stencils (quadratic nodes c..c+2, cubic c-1..c+3 per
                 // axis) span grid blocks (c-1)/4 .. (c+3)/4: marked whatever the

@@ -42,6 +42,7 @@ constexpr int kUnitX = 4, kUnitY = 4, kUnitZ = 8;
 constexpr int kQRows = kUnitY + 2, kQCols = kUnitZ + 2;   // nodes of a quadratic plane
 constexpr int kCRows = kUnitY + 4, kCCols = kUnitZ + 4;   // nodes of a cubic plane
 constexpr int kPlaneCols = 16;                // words of a plane row (see plane_word)
+constexpr int kFewCells = 2, kCloud = 24;     // below kCloud particles to a unit: layers of so few cells one by one
 constexpr int kRing = 4;                      // rows of a warp's ring, kRing - 1 on their way
 
 // Word of node (row, col) of a plane.  Odd rows are rotated by half: the 16
@@ -107,7 +108,7 @@ struct SweepShared {
     unsigned char split[kUnitCells];          // particles of the sub-block before the cell, mod 256
     int2 cell[kUnitCells];                    // {first place (kCellRows), particles}; regular cells only (0 otherwise)
     int2 raw[kUnitCells];                     // the next unit's cells
-    int layer_rows[kUnitX];
+    int layer_rows[kUnitX];                   // rows of a layer; negative: at most kFewCells cells (see sweep_layer)
     float dx;
     float scale[4];                           // fixed-point scales of {momentum, mass, w d, w}
     long long *g_quad, *g_cubic;              // global sums of the first node of the unit's plane 0
@@ -141,6 +142,12 @@ __device__ __forceinline__ int2 sweep_item(unsigned i, SweepItems n) {
 __device__ __forceinline__ int2 sweep_unit(unsigned i, SweepItems n, const int *__restrict__ work) {   // {unit, layers}
     const int2 item = sweep_item(i, n);
     return make_int2(item.x >= 0 ? work[item.x] : -1, item.y);
+}
+
+// SweepShared::layer_rows of a layer, cnt: this lane's cell.
+__device__ __forceinline__ int layer_code(int cnt, bool cloud) {
+    const int rows = __reduce_max_sync(0xffffffffu, cnt), cells = __popc(__ballot_sync(0xffffffffu, cnt > 0));
+    return cloud && cells <= kFewCells ? -rows : rows;
 }
 
 // Starts the copy of a particle's payload (src: its part 0) into this lane's
@@ -438,10 +445,14 @@ struct CubicLapSums {
 
 // Adds the rows of one layer (this lane's cell: `cell`, and `split`, see
 // SweepShared) to a warp's sums.  IN_ROWS: the layer's layout, known for the
-// whole layer.
+// whole layer.  few: the layer's sums go to the plane here, cell by cell with the
+// nodes over the lanes, not with the cells over the lanes node by node (add): a
+// cloud of 100k particles, 7 to a unit, 566 us per substep and 484.  (Only in
+// clouds: for the thin layers of bodies' surfaces it is the longer chain, 12 small
+// scenes 340 and 344 us.)
 template <bool IN_ROWS, class SUMS>
 __device__ __forceinline__ void sweep_layer(SweepShared &sh, SUMS &sums, typename SUMS::Slot *ring, const char *payload,
-                                            int2 cell, int split, int rows, int ox, int wid, int lane) {
+                                            int2 cell, int split, int rows, bool few, int ox, int wid, int lane) {
     const int first = cell.x & ~kCellRows;
     const float dx = sh.dx;
     // in rows the place's number in its block is the lane
@@ -473,9 +484,11 @@ __device__ __forceinline__ void sweep_layer(SweepShared &sh, SUMS &sums, typenam
             if (k + kRing - 1 < rows) copy(k + kRing - 1);   // into the slot of the row before this one
             cp_async_commit();
         }
-        if (k >= rows) break;
-        const bool mine = restart == k;
+        const bool end = k >= rows;
+        if (end && (IN_ROWS || !few)) break;     // (a layer in rows has at least 16 cells)
+        const bool mine = end ? cell.y > 0 : restart == k;
         for (unsigned m = __ballot_sync(0xffffffffu, mine); m; m &= m - 1) sums.add_lane(sh, wid, lane, __ffs(m) - 1);
+        if (end) break;
         if (mine) restart += 256;
     }
 }
@@ -492,15 +505,17 @@ __device__ __forceinline__ void sweep_warp(SweepShared &sh, typename SUMS::Slot 
     int ox = (set + 4 * N - x0) % N;                       // this warp's plane: X = x + ox
 #pragma unroll 1
     for (int x = x0; x < x1; ++x) {
-        const int rows = __reduce_max_sync(0xffffffffu, sh.layer_rows[x]);
-        if (rows > 0) {
+        const int code = __reduce_max_sync(0xffffffffu, sh.layer_rows[x]);
+        if (code != 0) {
+            const bool few = code < 0;
+            const int rows = abs(code);
             const int2 cell = sh.cell[32 * x + lane];
             const int split = sh.split[32 * x + lane];
             if (__any_sync(0xffffffffu, cell.x < 0))
-                sweep_layer<true>(sh, sums, ring, payload, cell, split, rows, ox, wid, lane);
+                sweep_layer<true>(sh, sums, ring, payload, cell, split, rows, few, ox, wid, lane);
             else
-                sweep_layer<false>(sh, sums, ring, payload, cell, split, rows, ox, wid, lane);
-            sums.add(sh, wid, lane);
+                sweep_layer<false>(sh, sums, ring, payload, cell, split, rows, few, ox, wid, lane);
+            if (!few) sums.add(sh, wid, lane);
             dirty = true;
         }
         if (dirty && (ox == 0 || x == x1 - 1)) {           // no later layer reaches this plane

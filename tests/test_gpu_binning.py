@@ -13,6 +13,7 @@ from test_gpu_parity import _rot, run_pieces, ws_views
 from test_gpu_sweep import _cell, _sim
 import oracle as orc
 from peel_mpm_b200 import _lib, scenes
+import peel_mpm_b200.differentiable as dfx
 
 pytestmark = pytest.mark.gpu
 
@@ -80,3 +81,58 @@ def test_sums_at_the_border_of_single_layers(more):
     assert rel_l2(grids["grid_mv"], mom[:, :3]) < 1e-5
     for got, name in ((mom[:, 3], "grid_m"), (dmg[:, 0], "grid_dc"), (dmg[:, 1], "grid_dwc")):
         assert rel_l2(grids[name], got) < tol
+
+
+def _cloud():
+    """Fewer than 24 particles to a unit: layers of one and two cells add cell by cell, three go the general way; among
+    them cells of 256 and 300, which restart at 256."""
+    ng = 64
+    rng = np.random.default_rng(11)
+    c = rng.permutation(14 * 14 * 7)[:80]
+    c = np.stack([4 + 4 * (c // 98), 4 + 4 * (c // 7 % 14), 4 + 8 * (c % 7)], 1)
+    x = [_cell(rng, v, 256 if i == 0 else 300, ng) for i, v in enumerate(c[:2])]
+    for i, v in enumerate(c[2:]):
+        for k in range(1 + i % 3):                      # cells of one layer
+            x.append(_cell(rng, v + [0, k, 2 * k], 1 + i % 4, ng))
+    sc, state = _scene(ng, np.concatenate(x), 5)
+    assert sc.n < 24 * 80
+    F = np.einsum("nij,nj,nkj->nik", _rot(rng, sc.n), rng.uniform(0.9, 1.1, size=(sc.n, 3)), _rot(rng, sc.n))
+    state.update(F=F.astype(np.float32), C=rng.normal(size=(sc.n, 3, 3)).astype(np.float32))
+    return rng, sc, state
+
+
+def test_sums_of_a_cloud_match_the_oracle():
+    rng, sc, state = _cloud()
+    ora = orc.OracleSim(sc, np.float32)
+    for f, a in state.items():
+        getattr(ora, f)[:] = a
+    grids = ora.alloc_grids()
+    ora.substep(0.0, grids=grids)
+    sim = _sim(sc, state)
+    run_pieces(sim, 0.0, ("bin", "p2g"))
+    w = ws_views(sim)
+    mom, dmg = w["g_mom"].cpu().numpy().astype(np.float64), w["g_dmg"].cpu().numpy().astype(np.float64)
+    tol = 2 * (300 + 32) * 2.0 ** -24
+    assert rel_l2(grids["grid_mv"], mom[:, :3]) < max(1e-5, tol)
+    for got, name in ((mom[:, 3], "grid_m"), (dmg[:, 0], "grid_dc"), (dmg[:, 1], "grid_dwc")):
+        assert rel_l2(grids[name], got) < tol
+
+
+def test_vjp_of_a_cloud_matches_the_forward_differences():
+    rng, sc, state = _cloud()
+    w = torch.tensor(rng.normal(size=(sc.n, 3)), dtype=torch.float32, device="cuda:0")
+    wl = torch.tensor(rng.normal(size=sc.n), dtype=torch.float32, device="cuda:0")
+
+    def forward(v, d):
+        sim = _sim(sc, state)
+        sim.v[:], sim.d[:] = v, d
+        sim.substep(0.0)
+        return sim.v.double(), sim.lap.double()
+
+    u, d = torch.tensor(state["v"], device="cuda:0"), _sim(sc, state).d.clone()
+    got = dfx.substep_vjp(_sim(sc, state), 0.0, {"v": w})[0]["v"].double()
+    want = (w.double() * (forward(u, d)[0] - forward(0 * u, d)[0])).sum()
+    assert abs(float((got * u).sum() - want)) < 2e-5 * float(w.norm() * u.norm())
+    got = dfx.substep_vjp(_sim(sc, state), 0.0, {"lap": wl})[0]["d"].double()
+    want = (wl.double() * (forward(u, d)[1] - forward(u, 0 * d)[1])).sum()
+    assert abs(float((got * d).sum() - want)) < 2e-5 * float(wl.norm() * d.norm()) * 12 * sc.n_grid ** 2
