@@ -214,13 +214,10 @@ __global__ void __launch_bounds__(256) k_adj_pre(const pm_params prm, const Part
         fx[ax] = __fsub_rn(X, fb);
     }
     {
-        const long long at = iperm[p];
-        float4 *dst = (float4 *)pay_at(pay, at);
-        dst[0] = reg ? make_float4(fx[0], fx[1], fx[2], lb) : make_float4(xp[0], xp[1], xp[2], lb);
-        dst[32] = make_float4(vt[0], vt[1], vt[2], 0.0f);
-        dst[64] = make_float4(kc[0], kc[3], kc[1], kc[4]);
-        dst[96] = make_float4(kc[2], kc[5], kc[6], kc[7]);
-        *pay_az2(pay, at) = kc[8];
+        const float4 part[4] = {reg ? make_float4(fx[0], fx[1], fx[2], lb) : make_float4(xp[0], xp[1], xp[2], lb),
+                                make_float4(vt[0], vt[1], vt[2], 0.0f), make_float4(kc[0], kc[3], kc[1], kc[4]),
+                                make_float4(kc[2], kc[5], kc[6], kc[7])};
+        pay_store(pay, iperm[p], part, kc[8]);
     }
     // bounds of one node contribution: |w (vt + K Ct dpos)| with w <= 1,
     // |dpos| <= 1.5 dx per axis (the cubic stencil's quadratic part), and

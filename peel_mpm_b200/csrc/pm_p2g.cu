@@ -598,12 +598,10 @@ __global__ void __launch_bounds__(256, MINB) k_stress(const SC sc, const Parts P
 #pragma unroll
     for (int k = 0; k < 9; ++k) aff[k] = coeff * tau[k] + m * Cp[k];
     {
-        float4 *dst = (float4 *)pay_at(w.payload, s);
-        dst[0] = reg ? make_float4(fx[0], fx[1], fx[2], d_new) : make_float4(xp[0], xp[1], xp[2], d_new);
-        dst[32] = make_float4(m * v[0], m * v[1], m * v[2], m);
-        dst[64] = make_float4(aff[0], aff[3], aff[1], aff[4]);
-        dst[96] = make_float4(aff[2], aff[5], aff[6], aff[7]);
-        *pay_az2(w.payload, s) = aff[8];
+        const float4 part[4] = {reg ? make_float4(fx[0], fx[1], fx[2], d_new) : make_float4(xp[0], xp[1], xp[2], d_new),
+                                make_float4(m * v[0], m * v[1], m * v[2], m), make_float4(aff[0], aff[3], aff[1], aff[4]),
+                                make_float4(aff[2], aff[5], aff[6], aff[7])};
+        pay_store(w.payload, s, part, aff[8]);
     }
     {   // bounds of one node contribution: |w (m v + aff dpos)| with w <= 1 and |dpos| <= 1.5 dx per axis
         const float hx = 1.5f * (float)prm.dx;

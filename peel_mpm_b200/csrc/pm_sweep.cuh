@@ -77,14 +77,26 @@ __device__ __forceinline__ void cp_async_wait() {   // until at most N of this t
 //   {fx, d} {v, m} {a00, a10, a01, a11} {a02, a12, a20, a21} {a22}
 // node o of its quadratic stencil receives w (v + a (o - fx) dx) and w m, a node
 // of its cubic stencil w d and w (the adjoint: d times the Laplacian's weights).
-// In global memory in blocks of 32 places, part after part (one row of a layer
-// in the row layout).
+// In global memory in blocks of 32 places (one row of a layer in the row layout):
+// part 0 of all, parts 1 and 2 of each side by side, part 3, part 4.  A particle
+// whose neighbours in the state lie elsewhere thus writes four sectors: 1M
+// particles in no order 509 us per substep with part after part (five sectors),
+// 489 so; the regular slab's sweep, which reads whole rows either way, is the
+// same to 0.4%.  (Parts 0 and 1, 2 and 3 side by side, three sectors: 476, but
+// the cubic planes' warps, which read part 0 alone, make the slab 1.1% slower.)
 constexpr int kPayBlock = kPayBytes * 32;
-__device__ __forceinline__ char *pay_at(void *payload, long long place) {   // part 0; part k 512 bytes on
-    return (char *)payload + (place >> 5) * kPayBlock + (place & 31) * 16;
+__device__ __forceinline__ int pay_part(int k, int i) {   // byte of part k of the block's place i
+    return k == 0 ? 16 * i : (k == 3 ? 1536 + 16 * i : (k == 4 ? 2048 + 4 * i : 496 + 16 * k + 32 * i));
 }
-__device__ __forceinline__ float *pay_az2(void *payload, long long place) {
-    return (float *)((char *)payload + (place >> 5) * kPayBlock + 2048) + (place & 31);
+__device__ __forceinline__ char *pay_block(const void *payload, long long place) {
+    return (char *)payload + (place >> 5) * kPayBlock;
+}
+__device__ __forceinline__ void pay_store(void *payload, long long place, const float4 (&p)[4], float a22) {
+    char *b = pay_block(payload, place);
+    const int i = (int)(place & 31);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) *(float4 *)(b + pay_part(k, i)) = p[k];
+    *(float *)(b + pay_part(4, i)) = a22;
 }
 // Place of the k-th particle of a cell from its first place.
 __device__ __forceinline__ long long place_of(int first, int k) {
@@ -150,16 +162,16 @@ __device__ __forceinline__ int layer_code(int cnt, bool cloud) {
     return cloud && cells <= kFewCells ? -rows : rows;
 }
 
-// Starts the copy of a particle's payload (src: its part 0) into this lane's
-// words of a ring slot; lanes without a particle get zeros.
-__device__ __forceinline__ void row_copy(QuadSlot &s, const char *src, int az2, bool on, int lane) {
+// Starts the copy of the payload of a block's place i into this lane's words of a
+// ring slot; lanes without a particle get zeros.
+__device__ __forceinline__ void row_copy(QuadSlot &s, const char *block, int i, bool on, int lane) {
     const int bytes = on ? 16 : 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) cp_async16(&s.p[j][lane], src + 512 * j, bytes);
-    cp_async4(&s.az2[lane], src + az2, bytes >> 2);
+    for (int k = 0; k < 4; ++k) cp_async16(&s.p[k][lane], block + pay_part(k, i), bytes);
+    cp_async4(&s.az2[lane], block + pay_part(4, i), bytes >> 2);
 }
-__device__ __forceinline__ void row_copy(CubicSlot &s, const char *src, int, bool on, int lane) {
-    cp_async16(&s.p0[lane], src, on ? 16 : 0);
+__device__ __forceinline__ void row_copy(CubicSlot &s, const char *block, int i, bool on, int lane) {
+    cp_async16(&s.p0[lane], block + pay_part(0, i), on ? 16 : 0);
 }
 
 // Adds NC sums to a node's word (byte address `at`) in NC planes `stride` bytes apart.
@@ -455,17 +467,15 @@ __device__ __forceinline__ void sweep_layer(SweepShared &sh, SUMS &sums, typenam
                                             int2 cell, int split, int rows, bool few, int ox, int wid, int lane) {
     const int first = cell.x & ~kCellRows;
     const float dx = sh.dx;
-    // in rows the place's number in its block is the lane
-    const char *src = payload + (long long)(first >> 5) * kPayBlock + lane * 16;
+    const char *src = pay_block(payload, first);   // in rows: place k of the cell is the lane's of the k-th block on
     auto copy = [&](int k) {
         const bool on = k < cell.y;
         if (IN_ROWS) {
-            row_copy(ring[k & (kRing - 1)], src, 2048 - 12 * lane, on, lane);
+            row_copy(ring[k & (kRing - 1)], src, lane, on, lane);
             src += kPayBlock;
         } else {
             const int s = on ? first + k : 0;
-            row_copy(ring[k & (kRing - 1)], payload + (long long)(s >> 5) * kPayBlock + (s & 31) * 16,
-                     2048 - 12 * (s & 31), on, lane);
+            row_copy(ring[k & (kRing - 1)], pay_block(payload, s), s & 31, on, lane);
         }
     };
 #pragma unroll
@@ -583,12 +593,13 @@ __device__ __noinline__ void scatter_clamped(SweepShared &sh, const WS *w, const
             __syncwarp();                          // the run before is done with
             if (lane < n) {
                 const long long s = place_of(first, k0 + lane);
-                const float4 *p = (const float4 *)(payload + (s >> 5) * kPayBlock + (s & 31) * 16);
-                const float4 p0 = p[0];
+                const char *block = pay_block(payload, s);
+                const int i = (int)(s & 31);
+                const float4 p0 = *(const float4 *)(block + pay_part(0, i));
                 slot.p[0][lane] = p0;
 #pragma unroll
-                for (int j = 1; j < 4; ++j) slot.p[j][lane] = p[32 * j];
-                slot.az2[lane] = ((const float *)(payload + (s >> 5) * kPayBlock + 2048))[s & 31];
+                for (int k = 1; k < 4; ++k) slot.p[k][lane] = *(const float4 *)(block + pay_part(k, i));
+                slot.az2[lane] = *(const float *)(block + pay_part(4, i));
                 const float xp[3] = {p0.x, p0.y, p0.z};
 #pragma unroll
                 for (int a = 0; a < 3; ++a) {
