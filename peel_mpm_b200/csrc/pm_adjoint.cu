@@ -262,7 +262,6 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_adj_sweep(const __grid_con
     const int lane = tid & 31, wid = __reduce_max_sync(0xffffffffu, tid >> 5);
     const unsigned n_units = min(head->n_work, (unsigned)min(n, (long long)0x1fffffff));
     const SweepItems items = sweep_items(n_units);
-    const bool cloud = n < (long long)kCloud * n_units;
     const int ng = prm.n_grid, nb = sort_blocks_per_axis(ng);
     for (int i = tid; i < kSweepQ * 4 * kQRows * kPlaneCols; i += kSweepThreads) sh.qpl[0][0][i] = 0;
     for (int i = tid; i < kSweepC * 2 * kCRows * kPlaneCols; i += kSweepThreads) sh.cpl[0][0][i] = 0;
@@ -291,7 +290,7 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_adj_sweep(const __grid_con
             const int cnt = clamped_cell(g, ng) ? 0 : cell.y;
             sh.cell[tid] = make_int2(cell.x, cnt);
             sh.split[tid] = split[(long long)i * kUnitCells + tid];
-            const int code = layer_code(cnt, cloud);
+            const int code = layer_code(cnt, false);
             if (lane == 0) sh.layer_rows[wid] = code;
         }
         if (tid == kSweepThreads - 1) {
@@ -304,9 +303,9 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_adj_sweep(const __grid_con
         unsigned take = 0;                // the next item is taken while this one is swept
         if (tid == kSweepThreads - 1) take = gridDim.x + atomicAdd(&actl->work_next, 1u);
         if (wid < kSweepQ)
-            sweep_warp<QuadSums<true>, kSweepQ>(sh, sh.qring[wid], (const char *)pay, wid, wid, lane, x0, x1);
+            sweep_warp<QuadSums<true>, kSweepQ, false>(sh, sh.qring[wid], (const char *)pay, wid, wid, lane, x0, x1);
         else
-            sweep_warp<CubicLapSums, kSweepC>(sh, sh.cring[wid - kSweepQ], (const char *)pay, wid, wid - kSweepQ, lane, x0,
+            sweep_warp<CubicLapSums, kSweepC, false>(sh, sh.cring[wid - kSweepQ], (const char *)pay, wid, wid - kSweepQ, lane, x0,
                                              x1);
         if (tid == kSweepThreads - 1) sh.next = sweep_item(take, items);
         __syncthreads();

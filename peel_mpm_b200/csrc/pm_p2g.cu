@@ -755,9 +755,9 @@ __global__ void __launch_bounds__(kSweepThreads, 3) k_p2g_sweep(const __grid_con
             cp_async8(&sh.raw[tid], w.cells + (long long)next.x * kUnitCells + tid);
         cp_async_commit();
         if (wid < kSweepQ)
-            sweep_warp<QuadSums<false>, kSweepQ>(sh, sh.qring[wid], (const char *)w.payload, wid, wid, lane, x0, x1);
+            sweep_warp<QuadSums<false>, kSweepQ, true>(sh, sh.qring[wid], (const char *)w.payload, wid, wid, lane, x0, x1);
         else
-            sweep_warp<CubicSums, kSweepC>(sh, sh.cring[wid - kSweepQ], (const char *)w.payload, wid, wid - kSweepQ,
+            sweep_warp<CubicSums, kSweepC, true>(sh, sh.cring[wid - kSweepQ], (const char *)w.payload, wid, wid - kSweepQ,
                                              lane, x0, x1);
         if (tid < 64) {                   // the blocks this item is the first to touch join the list
             const bool fresh = was == 0;
