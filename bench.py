@@ -80,13 +80,13 @@ BYTES_PER_NODE = 80
 # `traffic` and its issue-bound floor (warp instructions / (4 schedulers x
 # SMs x SM clock)).
 NCU_KERNELS = {
-    "k_count": {"dram_bytes": 14887168, "warp_inst": 4003004},
-    "k_offsets": {"dram_bytes": 1429760, "warp_inst": 482551},
-    "k_place": {"dram_bytes": 18054400, "warp_inst": 3670016},
-    "k_rank": {"dram_bytes": 5716480, "warp_inst": 5091289},
-    "k_stress": {"dram_bytes": 195964928 + 51072768, "warp_inst": 39837552},
-    "k_p2g_sweep": {"dram_bytes": 81618176 + 1478656, "warp_inst": 66801624},
-    "k_g2p": {"dram_bytes": 54691328 + 45396480, "warp_inst": 48168960},
+    "k_count": {"dram_bytes": 14891776, "warp_inst": 4005605},
+    "k_offsets": {"dram_bytes": 1432064, "warp_inst": 594088},
+    "k_place": {"dram_bytes": 18053376, "warp_inst": 3670016},
+    "k_rank": {"dram_bytes": 5722112, "warp_inst": 5221769},
+    "k_stress": {"dram_bytes": 195639040 + 51587584, "warp_inst": 39903088},
+    "k_p2g_sweep": {"dram_bytes": 81604096 + 885248, "warp_inst": 68740280},
+    "k_g2p": {"dram_bytes": 54689280 + 45598208, "warp_inst": 48168960},
 }
 P2G_KERNELS = ("k_count", "k_offsets", "k_place", "k_rank", "k_stress", "k_p2g_sweep")
 LAUNCHES_PER_SUBSTEP = 3 + len(P2G_KERNELS)   # and clock, grid, g2p; one scene or a batch of any number

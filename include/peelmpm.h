@@ -193,7 +193,9 @@ int pm_set_clock(const pm_params *prm, void *ws, size_t ws_bytes, int64_t n, con
  * in particle order. */
 int pm_bin(const pm_params *prm, const pm_particles *P, void *ws, size_t ws_bytes, void *stream);
 /* Particle BCs, constitutive update, damage update, degradation, quadratic
- * P2G and cubic damage scatter (anisompm.py:601-724, 768-776). */
+ * P2G and cubic damage scatter (anisompm.py:601-724, 768-776).  A caller may
+ * stop here, to look at pm_grid_sums: later substeps find every block they
+ * touch.  The sums stay until a grid update, and a P2G before it adds to them. */
 int pm_p2g(const pm_params *prm, const pm_particles *P, void *ws, size_t ws_bytes, void *stream);
 /* Grid velocity update with gravity, damping, mask, colliders, and damage
  * field normalisation (anisompm.py:727-746, 777-779). */
@@ -233,8 +235,10 @@ typedef struct pm_param_adj {
 } pm_param_adj;
 
 /* Tape for `slots` recorded substeps of n particles on an n_grid^3 grid:
- * per slot 24 bytes per grid node and 124 bytes per particle, plus three
- * shared adjoint grids (48 bytes per node).  flags: PM_TAPE_COLLIDERS when the
+ * per slot 24 bytes per grid node, 132 bytes per particle and 1,156 bytes per
+ * unit of 4 x 4 x 8 cells that can be listed (at most one per particle), plus,
+ * shared by the slots, the adjoint's three grids (64 bytes per node) and its
+ * payload (136 bytes per particle).  flags: PM_TAPE_COLLIDERS when the
  * recorded substeps have grid colliders (each slot then also keeps the grid
  * velocity before the colliders, 16 bytes per node); pm_substep_record and
  * pm_substep_adjoint derive the layout from their pm_params and reject a

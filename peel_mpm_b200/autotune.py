@@ -30,7 +30,7 @@ from typing import Optional
 
 import torch
 
-P2G_CANDIDATES = (0, 2, 4)             # 0: as many as fit (3 per SM)
+P2G_CANDIDATES = (0, 2, 4)             # 0: as many as fit (3 per SM), and so 4: the same launch
 STRESS_CANDIDATES = (3, 4)
 G2P_CANDIDATES = (3, 4)
 GRID_CANDIDATES = (0, 4, 8, 16, 32)    # 0: one thread per node row

@@ -26,10 +26,13 @@
 // Morton order of its cells.  The sums of a substep are thus fixed by the
 // particles alone, not by the order of arrival, the launch or the batch.
 //
-// Bound by instruction issue (64%) and the FMA pipe.  1M displaced particles, 6 to
-// 11 per cell: 133 us, the former tile kernel 129.  It gains where cells hold more
-// or units are few: with the counted binning 8.8M particles at 27 per cell go from
-// 6,360 to 5,250 us per two substeps, 138k from 1,227 to 597 us per six.
+// Bound by instruction issue (68%) and the FMA pipe.  1M displaced particles, 6 to
+// 11 per cell: 114 us, the former tile kernel 129; on a regular lattice of 8 per
+// cell 102 and 99.5, and below 2 per cell it is the slower one too (a layer's sums
+// go to the planes for all 32 cells: 885k at 1 per cell 332 us and 280).  It gains
+// where cells hold more or units are few: with the counted binning 8.8M particles at
+// 27 per cell go from 6,400 to 5,090 us per two substeps, 138k from 1,205 to 598
+// us per six.
 #pragma once
 
 #include "pm_common.cuh"
